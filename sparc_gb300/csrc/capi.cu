@@ -381,7 +381,7 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     c->use_graphs = getenv("SPARC_NO_GRAPHS") == nullptr && !mhd_form;
     if (c->use_fused) {
         fused_prepare(c->nz, c->nzpml);
-        if ((rc = dalloc(c, &c->src_plane, (size_t)c->S * c->M * 8))) return bail(rc);
+        if ((rc = dalloc(c, &c->src_plane, (size_t)FUSED_STEPS * c->S * c->M * 8))) return bail(rc);
     }
     if (mhd_form && (rc = mhd_create(c))) return bail(rc);
     // twiddles cos/sin(2 pi q / n), q < n/2, exact pi; the FP32 copy (rounded
@@ -1001,27 +1001,34 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
         Fz.pf_stride = 1;
         Fz.src_plane = (float2*)c->src_plane;
         Fz.wait_limit = c->fused_test_nocopy ? 64 : (1 << 22);
-    }
-    for (int it = 0; it < nsteps; ++it) {
-        if (fused) {
-            Fz.write_scr = (it == nsteps - 1 && c->rhs_out) ? 1 : 0;
+        if (c->rec_on) {
+            Fz.rec = (float2*)c->rec; Fz.rec_steps = c->steps; Fz.rec_max = c->rec_max; Fz.rec_k = c->o_rad - 1;
+        }
+        // a pencil's step needs nothing of another pencil, so one launch takes up
+        // to FUSED_STEPS steps of every pencil with its state on chip
+        for (int it = 0; it < nsteps; it += Fz.nsteps) {
+            Fz.nsteps = std::min(nsteps - it, FUSED_STEPS);
+            Fz.write_scr = (it + Fz.nsteps == nsteps && c->rhs_out) ? 1 : 0;
             if (Fz.src_mode == 2) {
                 launch_source_plane(Fz, c->active_n, c->stream);
                 c->launches += 1;
             }
             launch_fused(Fz, c->active_n, c->stream);
-            c->launches += 1;
-            CKL();
-        } else {
-            for (int rk = 0; rk < 5; ++rk) {
-                A.beta = (T)c->betas[rk];
-                A.has_scr = (rk > 0);
-                launch_stage<T>(A, c->active_n, c->stream);
-            }
-            launch_update<T>(U, c->active_n, c->stream);
-            c->launches += 6;
+            launch_tick(c->d_time, Fz.nsteps, c->stream);
+            c->launches += 2;
             CKL();
         }
+        return SPARC_OK;
+    }
+    for (int it = 0; it < nsteps; ++it) {
+        for (int rk = 0; rk < 5; ++rk) {
+            A.beta = (T)c->betas[rk];
+            A.has_scr = (rk > 0);
+            launch_stage<T>(A, c->active_n, c->stream);
+        }
+        launch_update<T>(U, c->active_n, c->stream);
+        c->launches += 6;
+        CKL();
         if (c->rec_on) {
             // v_z: field 6 of the displacement forms, field 4 of the velocity form
             launch_record<T>(CP<T>(c->a), CP<T>(c->rec), c->d_t0, c->d_time, c->steps, c->rec_max, c->fs, c->M,
@@ -1029,7 +1036,7 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
             c->launches++;
             CKL();
         }
-        launch_tick(c->d_time, c->stream);
+        launch_tick(c->d_time, 1, c->stream);
         c->launches++;
         CKL();
     }

@@ -1,12 +1,13 @@
 // Fused FP32 time step: the five LDDRK stages, the update, the z filter and
-// the horizontal filter of one time step in a single kernel, with the state
-// of each z-pencil held on chip for the whole step.
+// the horizontal filter of up to FUSED_STEPS time steps in a single kernel,
+// with the state of each z-pencil held on chip from step to step.
 //
 // Work decomposition.  A work item is P = 2, 4 or 8 consecutive horizontal
-// modes m of one source; the launch has one CTA per resident slot (one per SM
-// at P = 8), and CTA b takes items b, b + G, b + 2G, ... (G CTAs), loading the
-// z tables once and issuing each item's tile copies right after the previous
-// item's stores have read the tile out of shared memory.  Each mode's
+// modes m of one source.  A launch of one step has one CTA per resident slot
+// (one per SM at P = 8), and CTA b takes items b, b + G, b + 2G, ... (G CTAs),
+// loading the z tables once and issuing each item's tile copies right after
+// the previous item's stores have read the tile out of shared memory; a launch
+// of several steps has one CTA per item.  Each mode's
 // z-pencil is split into chunks of CH = 5 levels, one chunk per thread:
 // TP = 32*W threads per pencil, W = ceil(nz / 160) warps, and the pencil is
 // padded to NZP = TP*CH levels.
@@ -53,7 +54,14 @@
 //   * a LAGRANGE_INTERP source (the adjoint's) is interpolated to the step by
 //     a small kernel launched before it (source_plane_kernel), so no CTA
 //     spends its critical path on the seven FP64 weights.
-// HBM traffic per step: read a, write a (+ the PML planes and source planes),
+//   * a pencil's step needs nothing of another pencil, so a launch takes up
+//     to FUSED_STEPS = 16 steps before the tile goes back to HBM.  Loading and
+//     storing the tile, and the z tables, took a quarter of a CTA's time when
+//     every step did it.  Measured per step: 256x256x300, 8 sources 5.55 ->
+//     4.19 ms; 512x512x300, one adjoint source 2.99 -> 2.10 ms; results bit
+//     for bit the same.  The limit bounds a CTA's time (about half a
+//     millisecond), after which launches of other streams get its SM.
+// HBM traffic per launch: read a, write a (+ the PML planes and source planes),
 // and scr only on steps whose right-hand side is requested (outputs).
 #include <algorithm>
 #include <type_traits>
@@ -299,15 +307,6 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
         float2* gP = A.pml + (long long)s * 2 * A.ps;
         // 16 B vector copies need every row start z*M + m0 to be even (M even)
         const bool vec = ((M & 1) == 0) && (m0 + P <= M);
-        if (!first) {
-            // the previous item's update and filter wrote the padding levels
-            // nz..NZP-1 of every row: zero them again
-            const int np = NZP - nz;
-            for (int r = threadIdx.x; r < 6 * P * np; r += nthr) {
-                const int row = r / np, k = r - row * np;
-                tile[row * LZ + GZ + nz + k] = make_float2(0.f, 0.f);
-            }
-        }
         // ---- load the a tile and the PML tile: every complex value by its own
         // asynchronous 8-byte copy into its transposed place, all in flight at
         // once ([z][m] in HBM, [mode][z] on chip), awaited with the z tables ----
@@ -343,8 +342,7 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
                 }
             }
         }
-        const int tl = *A.clk.time - A.clk.t0[s];           // this slot's clock
-        const bool src_on = A.src_mode != 0 && slot_src_on(A.clk, tl);
+        const int tl0 = *A.clk.time - A.clk.t0[s];          // this slot's clock at the first step
         // this mode's multipliers, loaded while the tile copies are in flight
         const float kx = mvalid ? A.pt[PT_KX * M + m] : 0.f;
         const float ky = mvalid ? A.pt[PT_KY * M + m] : 0.f;
@@ -400,19 +398,6 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
             }
         }
         const bool pml_t = pmask != 0;
-        const bool src_t = src_on && mvalid && A.ksrc >= j0 && A.ksrc < j0 + CH;
-        // forcing of this step for this mode (only the thread owning the source plane uses it)
-        float2 F = make_float2(0.f, 0.f);
-        if (src_t) {
-            if (A.src_mode == 1) {
-                const float2* pl = A.planes + (long long)s * A.plane_ss + m;
-                float w = (tl < A.nseries) ? (float)A.series[(long long)s * A.nseries + tl] : 0.f;
-                F = w * pl[0];
-            } else {   // this step's interpolated plane, from source_plane_kernel
-                F = A.src_plane[(long long)s * M + m];
-            }
-            F = A.src_scale * F;
-        }
 
         float2 sc[6][CH];
         #pragma unroll
@@ -424,6 +409,10 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
         auto TA = [&](int f, int j) -> float2 { return tp[f * P * LZ + j]; };
         // z table entry of row r at level j, as a pair
         auto Z2 = [&](int r, int j) { return zt2(zs, r * NZP + j); };
+
+        // forcing of a step for this mode (only the thread owning the source plane uses it)
+        float2 F = make_float2(0.f, 0.f);
+        bool src_t = false;
 
         // one LDDRK stage; HS: the stage argument is a + beta*scr (stages 2-5)
         // rather than a (stage 1), fixed at compile time
@@ -545,79 +534,108 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
                     if (j0 + q == nz - 1) sc[5][q] = sc[2][q] = make_float2(0.f, 0.f);
             }
         };
-        stage(std::integral_constant<bool, false>(), 0.f);
-        for (int rk = 1; rk < 5; ++rk) {
-            // static parameter indices keep the argument block out of local memory
-            const float beta = rk == 1 ? A.betas[1] : rk == 2 ? A.betas[2] : rk == 3 ? A.betas[3] : A.betas[4];
-            stage(std::integral_constant<bool, true>(), beta);
-        }
-
-        // ---- update a += dt*scr, pml += dt*scrpml (step.f90:114-116) ----
-        const float dt = A.dt;
-        const float2 DT = bc2(dt);
-        #pragma unroll
-        for (int f = 0; f < 6; ++f)
-            #pragma unroll
-            for (int q = 0; q < CH; ++q) {
-                float2* a = tp + f * P * LZ + j0 + q;
-                *a = pfma(DT, sc[f][q], *a);
-            }
-        if (pml_t) {
-            #pragma unroll
-            for (int q = 0; q < CH; ++q) {
-                if (pmask & (1u << q)) {
-                    const int ip = pipv + q;
-                    ptile[ip * P + pi] = ptile[ip * P + pi] + dt * spt[ip * P + pi];
-                    ptile[(nzpml + ip) * P + pi] = ptile[(nzpml + ip) * P + pi] + dt * spt[(nzpml + ip) * P + pi];
+        // ---- the launch's time steps: the pencil stays on chip from one to the
+        // next, and goes back to HBM after the last ----
+        #pragma unroll 1
+        for (int step = 0; step < A.nsteps; ++step) {
+            const int tl = tl0 + step;
+            src_t = A.src_mode != 0 && slot_src_on(A.clk, tl) && mvalid && A.ksrc >= j0 && A.ksrc < j0 + CH;
+            if (src_t) {
+                if (A.src_mode == 1) {
+                    const float2* pl = A.planes + (long long)s * A.plane_ss + m;
+                    float w = (tl < A.nseries) ? (float)A.series[(long long)s * A.nseries + tl] : 0.f;
+                    F = w * pl[0];
+                } else {   // this step's interpolated plane, from source_plane_kernel
+                    F = A.src_plane[((long long)step * A.nsrc + s) * M + m];
                 }
+                F = A.src_scale * F;
             }
-        }
-        pencil_sync(pi, TP);
-        // ---- z filter (+ horizontal filter): field f is filtered into registers,
-        // and written back after the next barrier, while field f+1 is filtered ----
-        const float hf = mvalid ? A.pt[PT_HF * M + m] : 1.f;
-        const float h1 = 0.5f * 0.41015625f, h2 = 0.5f * -0.234375f, h3 = 0.5f * 0.087890625f;
-        const float h4 = 0.5f * -0.01953125f, h5 = 0.5f * 0.001953125f, c0 = 0.75390625f;
-        const bool hfil_on = slot_hfilter(A.clk, tl);
-        const bool flo = j0 < 5, fhi = (j0 < nz) && (j0 + CH > nz - 5);
-        float2 prev[CH];
-        #pragma unroll
-        for (int f = 0; f < 7; ++f) {
-            float2 out[CH];
-            if (f < 6) {
-                const float2* V = tp + f * P * LZ;
+            stage(std::integral_constant<bool, false>(), 0.f);
+            #pragma unroll 1
+            for (int rk = 1; rk < 5; ++rk) {
+                // static parameter indices keep the argument block out of local memory
+                const float beta = rk == 1 ? A.betas[1] : rk == 2 ? A.betas[2] : rk == 3 ? A.betas[3] : A.betas[4];
+                stage(std::integral_constant<bool, true>(), beta);
+            }
+
+            // ---- update a += dt*scr, pml += dt*scrpml (step.f90:114-116) ----
+            const float dt = A.dt;
+            const float2 DT = bc2(dt);
+            #pragma unroll
+            for (int f = 0; f < 6; ++f)
                 #pragma unroll
                 for (int q = 0; q < CH; ++q) {
-                    const int j = j0 + q;
-                    float2 acc = pmul(bc2(c0), V[j]);
-                    acc = pfma(bc2(h1), padd(V[j - 1], V[j + 1]), acc);
-                    acc = pfma(bc2(h2), padd(V[j - 2], V[j + 2]), acc);
-                    acc = pfma(bc2(h3), padd(V[j - 3], V[j + 3]), acc);
-                    acc = pfma(bc2(h4), padd(V[j - 4], V[j + 4]), acc);
-                    out[q] = pfma(bc2(h5), padd(V[j - 5], V[j + 5]), acc);
+                    float2* a = tp + f * P * LZ + j0 + q;
+                    *a = pfma(DT, sc[f][q], *a);
                 }
-                if (flo || fhi) {   // FILTER_VARS_3D / _2D boundary rows
+            if (pml_t) {
+                #pragma unroll
+                for (int q = 0; q < CH; ++q) {
+                    if (pmask & (1u << q)) {
+                        const int ip = pipv + q;
+                        ptile[ip * P + pi] = ptile[ip * P + pi] + dt * spt[ip * P + pi];
+                        ptile[(nzpml + ip) * P + pi] = ptile[(nzpml + ip) * P + pi] + dt * spt[(nzpml + ip) * P + pi];
+                    }
+                }
+            }
+            pencil_sync(pi, TP);
+            // ---- z filter (+ horizontal filter): field f is filtered into registers,
+            // and written back after the next barrier, while field f+1 is filtered ----
+            const float h1 = 0.5f * 0.41015625f, h2 = 0.5f * -0.234375f, h3 = 0.5f * 0.087890625f;
+            const float h4 = 0.5f * -0.01953125f, h5 = 0.5f * 0.001953125f, c0 = 0.75390625f;
+            const bool hfil_on = slot_hfilter(A.clk, tl);
+            const float hf = (hfil_on && mvalid) ? A.pt[PT_HF * M + m] : 1.f;
+            const bool flo = j0 < 5, fhi = (j0 < nz) && (j0 + CH > nz - 5);
+            float2 prev[CH];
+            #pragma unroll
+            for (int f = 0; f < 7; ++f) {
+                float2 out[CH];
+                if (f < 6) {
+                    const float2* V = tp + f * P * LZ;
                     #pragma unroll
                     for (int q = 0; q < CH; ++q) {
                         const int j = j0 + q;
-                        const bool near_bot = (j >= 1 && j <= 4), near_top = (j >= nz - 5 && j <= nz - 2);
-                        if (j == 0 || j == nz - 1) out[q] = V[j];
-                        else if (near_top) out[q] = 0.5f * (V[j + 1] + V[j - 1]);
-                        else if (near_bot) out[q] = D3 ? 0.5f * (V[j + 1] + V[j - 1]) : V[j];
+                        float2 acc = pmul(bc2(c0), V[j]);
+                        acc = pfma(bc2(h1), padd(V[j - 1], V[j + 1]), acc);
+                        acc = pfma(bc2(h2), padd(V[j - 2], V[j + 2]), acc);
+                        acc = pfma(bc2(h3), padd(V[j - 3], V[j + 3]), acc);
+                        acc = pfma(bc2(h4), padd(V[j - 4], V[j + 4]), acc);
+                        out[q] = pfma(bc2(h5), padd(V[j - 5], V[j + 5]), acc);
+                    }
+                    if (flo || fhi) {   // FILTER_VARS_3D / _2D boundary rows
+                        #pragma unroll
+                        for (int q = 0; q < CH; ++q) {
+                            const int j = j0 + q;
+                            const bool near_bot = (j >= 1 && j <= 4), near_top = (j >= nz - 5 && j <= nz - 2);
+                            if (j == 0 || j == nz - 1) out[q] = V[j];
+                            else if (near_top) out[q] = 0.5f * (V[j + 1] + V[j - 1]);
+                            else if (near_bot) out[q] = D3 ? 0.5f * (V[j + 1] + V[j - 1]) : V[j];
+                        }
+                    }
+                    if (hfil_on && (D3 ? (f < 5) : true)) {
+                        #pragma unroll
+                        for (int q = 0; q < CH; ++q) out[q] = hf * out[q];
                     }
                 }
-                if (hfil_on && (D3 ? (f < 5) : true)) {
+                if (f < 6 && j0 + CH > nz) {   // the padding levels stay zero for the next step
                     #pragma unroll
-                    for (int q = 0; q < CH; ++q) out[q] = hf * out[q];
+                    for (int q = 0; q < CH; ++q)
+                        if (j0 + q >= nz) out[q] = make_float2(0.f, 0.f);
                 }
-            }
-            if (f > 0) {
-                pencil_sync(pi, TP);   // every thread has read field f-1's neighbours
+                if (f > 0) {
+                    pencil_sync(pi, TP);   // every thread has read field f-1's neighbours
+                    #pragma unroll
+                    for (int q = 0; q < CH; ++q) tp[(f - 1) * P * LZ + j0 + q] = prev[q];
+                }
                 #pragma unroll
-                for (int q = 0; q < CH; ++q) tp[(f - 1) * P * LZ + j0 + q] = prev[q];
+                for (int q = 0; q < CH; ++q) prev[q] = out[q];
             }
-            #pragma unroll
-            for (int q = 0; q < CH; ++q) prev[q] = out[q];
+            // surface record: v_z on the observation plane after a step on the
+            // slot's output cadence (driver.f90:455-476)
+            if (A.rec && mvalid && tl >= 0 && tl % A.rec_steps == 0 && A.rec_k >= j0 && A.rec_k < j0 + CH) {
+                const int r = tl / A.rec_steps;
+                if (r < A.rec_max) A.rec[((long long)s * A.rec_max + r) * M + m] = TA(5, A.rec_k);
+            }
         }
         __syncthreads();   // the store below copies every pencil's rows
         // ---- store a and the PML planes.  A row [f][z] of the CTA's P modes is
@@ -659,7 +677,8 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
             #pragma unroll
             for (int f = 0; f < 6; ++f)
                 #pragma unroll
-                for (int q = 0; q < CH; ++q) tp[f * P * LZ + j0 + q] = sc[f][q];
+                for (int q = 0; q < CH; ++q)
+                    if (j0 + q < nz) tp[f * P * LZ + j0 + q] = sc[f][q];
             __syncthreads();
             store_rows(gS);
         }
@@ -673,14 +692,15 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
 // of every slot interpolated to the step about to run, sum over l of
 // w(l) * vr(l) with the FP64 weights of the slot's clock (samples that take
 // no part have weight 0 and are skipped), in FP32 in the order of l.  One
-// launch before each fused step, so that the step's CTAs read one value
-// instead of each computing the seven FP64 weights on its critical path.
+// launch before each fused launch, for all its steps (grid.z), so that the
+// step's CTAs read one value instead of each computing the seven FP64 weights
+// on its critical path.
 __global__ void __launch_bounds__(256) source_plane_kernel(const FusedArgs A) {
     __shared__ double w[8];
     __shared__ int id[8];
     const int s = blockIdx.y;
     if (threadIdx.x < 7) {
-        const int tl = *A.clk.time - A.clk.t0[s];
+        const int tl = *A.clk.time - A.clk.t0[s] + (int)blockIdx.z;
         int i;
         const double v = lagrange_weight(A.clk, tl, A.L, threadIdx.x, &i);
         w[threadIdx.x] = v;
@@ -694,11 +714,13 @@ __global__ void __launch_bounds__(256) source_plane_kernel(const FusedArgs A) {
     #pragma unroll
     for (int l = 0; l < 7; ++l)
         if (w[l] != 0.0) F = F + (float)w[l] * pl[(long long)id[l] * A.M];
-    A.src_plane[(long long)s * A.M + m] = F;
+    A.src_plane[((long long)blockIdx.z * A.nsrc + s) * A.M + m] = F;
 }
 
 void launch_source_plane(const FusedArgs& A, int nsrc, cudaStream_t s) {
-    source_plane_kernel<<<dim3((A.M + 255) / 256, nsrc), 256, 0, s>>>(A);
+    FusedArgs B = A;
+    B.nsrc = nsrc;
+    source_plane_kernel<<<dim3((A.M + 255) / 256, nsrc, A.nsteps), 256, 0, s>>>(B);
 }
 
 int fused_w(int nz) { return (nz + 32 * CH - 1) / (32 * CH); }
@@ -748,7 +770,10 @@ static void launch_fused_t(const FusedArgs& A, int nsrc, cudaStream_t s) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fused_step_kernel<D3, W, P>, P * 32 * W, sm);
     const long long items = (long long)((A.M + P - 1) / P) * nsrc;
     const long long resident = (long long)std::max(nsm, 1) * std::max(occ, 1);
-    const int ncta = (int)std::min(items, resident);
+    // one step: one CTA per resident slot, looping over the items (its z tables
+    // are loaded once).  Several steps: one CTA per item, so that a launch of
+    // another stream gets SMs as the items end.
+    const int ncta = (int)(A.nsteps > 1 ? items : std::min(items, resident));
     fused_step_kernel<D3, W, P><<<ncta, P * 32 * W, sm, s>>>(B);
 }
 

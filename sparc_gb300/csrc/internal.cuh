@@ -381,12 +381,16 @@ struct FusedArgs {
     int* err;           // set to 1 if the bounded wait for the z-table bulk copy gave up
     int wait_limit;     // polls of that wait before it gives up
     int no_copy;        // test switch: issue no bulk copy, so the wait runs out with nothing in flight
-    float2* src_plane;  // [S][M] this step's interpolated source plane (src_mode 2, source_plane_kernel)
+    float2* src_plane;  // [nsteps][nsrc][M] each step's interpolated source plane (src_mode 2, source_plane_kernel)
+    int nsteps;         // time steps of the launch, at most FUSED_STEPS
+    float2* rec;        // surface records [S][rec_max][M], or null: v_z at level rec_k every rec_steps steps
+    int rec_steps, rec_max, rec_k;
     int nsrc;           // sources of the launch (set by the launcher)
     int pf_stride;      // > 0: each CTA prefetches into L2 the rows of the CTA pf_stride later in launch
                         // order (set by the launcher to the CTAs resident at once); 0: no prefetch
 };
 constexpr int FUSED_CH = 5;
+constexpr int FUSED_STEPS = 16;   // time steps of one launch of the fused step, at most
 void fused_prepare(int nz, int nzpml);
 size_t fused_smem_bytes(int nz, int nzpml, int W);
 bool fused_fits(int P, int nz, int nzpml);
@@ -403,9 +407,9 @@ template <typename T> void launch_update(const UpdateArgs<T>& A, int nsrc, cudaS
 template <typename T>
 void launch_record(const typename CplxOf<T>::type* a, typename CplxOf<T>::type* rec, const int* t0, const int* time,
                    int steps, int rec_max, long long fs, int M, int kplane, int field, int nsrc, cudaStream_t s);
-// the device time counter: set, and advance by one step
+// the device time counter: set, and advance by n steps
 void launch_set_time(int* time, int value, cudaStream_t s);
-void launch_tick(int* time, cudaStream_t s);
+void launch_tick(int* time, int n, cudaStream_t s);
 template <typename T>
 void launch_zderiv(const T* zt, const Compact<T>& cc, const typename CplxOf<T>::type* in,
                    typename CplxOf<T>::type* out, long long n1, int nz, int bc, int filter,

@@ -2025,7 +2025,7 @@ int mhd_steps_t(sparc_ctx* c, int nsteps) {
             c->launches++;
             CKL();
         }
-        launch_tick(c->d_time, c->stream);
+        launch_tick(c->d_time, 1, c->stream);
         c->launches++;
         CKL();
         c->time++;

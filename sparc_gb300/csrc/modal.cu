@@ -724,11 +724,11 @@ template void launch_record<float>(const float2*, float2*, const int*, const int
 
 // The context's time lives on the device so that a captured sequence of
 // steps replays at any time: the step kernels read it, and one thread
-// advances it after each step.
+// advances it after each launch of steps.
 __global__ void set_time_kernel(int* time, int value) { *time = value; }
-__global__ void tick_kernel(int* time) { *time = *time + 1; }
+__global__ void tick_kernel(int* time, int n) { *time = *time + n; }
 void launch_set_time(int* time, int value, cudaStream_t s) { set_time_kernel<<<1, 1, 0, s>>>(time, value); }
-void launch_tick(int* time, cudaStream_t s) { tick_kernel<<<1, 1, 0, s>>>(time); }
+void launch_tick(int* time, int n, cudaStream_t s) { tick_kernel<<<1, 1, 0, s>>>(time, n); }
 
 template <typename T> void launch_stage(const StageArgs<T>& A, int nsrc, cudaStream_t s) {
     const int b = A.block == 32 ? 32 : A.block == 64 ? 64 : 128;
