@@ -1,6 +1,6 @@
 """Build libsparc_gpu.so in-tree with nvcc for sm_103a (GB300).
 
-The three translation units compile in parallel, then link into
+The translation units compile in parallel, then link into
 ``sparc_gb300/_lib/libsparc_gpu.so``.  No PyTorch or cmake is involved; the
 library depends on the CUDA runtime only.
 """
@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libsparc_gpu.so")
-SOURCES = ["capi.cu", "modal.cu", "fft.cu", "noalloc.cu", "fused.cu", "mhd.cu", "adjsrc.cu", "update.cu"]
+SOURCES = ["capi.cu", "modal.cu", "fft.cu", "noalloc.cu", "fused.cu", "pencil.cu", "mhd.cu", "adjsrc.cu", "update.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 

@@ -69,14 +69,14 @@ Tri tri_for(int nz, int ibc) {
     return t;
 }
 
-// Elimination rows of the fused step for boundary code ibc (FP64): 1/betad,
+// Elimination rows of the whole-step kernels for boundary code ibc (FP64): 1/betad,
 // the forward multipliers m, their products H from each chunk's first level,
 // the backward multipliers g and their products G from each chunk's last
-// level (chunks of FUSED_CH levels; padding levels up to nzp are zero).
+// level (chunks of ch levels; padding levels up to nzp are zero).
 struct FusedRows {
     std::vector<double> ibd, mm, HH, gg, GG;
 };
-FusedRows fused_rows(int nz, int nzp, const Tri& t) {
+FusedRows fused_rows(int nz, int nzp, const Tri& t, int ch = FUSED_CH) {
     FusedRows r;
     r.ibd.assign(nzp, 0.0); r.mm.assign(nzp, 0.0); r.gg.assign(nzp, 0.0); r.HH.assign(nzp, 0.0);
     r.GG.assign(nzp, 0.0);
@@ -85,8 +85,8 @@ FusedRows fused_rows(int nz, int nzp, const Tri& t) {
         r.mm[j] = (j == 0) ? 0.0 : -t.low[j] / t.betad[j];
         r.gg[j] = (j == nz - 1) ? 0.0 : -t.gam[j + 1];
     }
-    for (int j0 = 0; j0 < nzp; j0 += FUSED_CH) {
-        const int j1 = j0 + FUSED_CH;
+    for (int j0 = 0; j0 < nzp; j0 += ch) {
+        const int j1 = j0 + ch;
         double pr = 1.0;
         for (int j = j0; j < j1; ++j) { pr *= r.mm[j]; r.HH[j] = pr; }
         pr = 1.0;
@@ -100,7 +100,7 @@ FusedRows fused_rows(int nz, int nzp, const Tri& t) {
 // sig(j)/sig(j-1); back substitution y(j) = sig(j) u(j) + g(j) sig(j)/sig(j+1)
 // y(j+1); the chunk products H, G are those of the new multipliers.  Same
 // recurrences, the scale applied inside them (sig = 1 on padding levels).
-FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig) {
+FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig, int ch = FUSED_CH) {
     FusedRows o = r;
     const int nzp = (int)r.ibd.size();
     for (int j = 0; j < nzp; ++j) {
@@ -108,8 +108,8 @@ FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig) 
         o.mm[j] = (j == 0) ? r.mm[j] : r.mm[j] * sig[j] / sig[j - 1];
         o.gg[j] = (j == nzp - 1) ? r.gg[j] : r.gg[j] * sig[j] / sig[j + 1];
     }
-    for (int j0 = 0; j0 < nzp; j0 += FUSED_CH) {
-        const int j1 = j0 + FUSED_CH;
+    for (int j0 = 0; j0 < nzp; j0 += ch) {
+        const int j1 = j0 + ch;
         double pr = 1.0;
         for (int j = j0; j < j1; ++j) { pr *= o.mm[j]; o.HH[j] = pr; }
         pr = 1.0;
@@ -122,11 +122,11 @@ FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig) 
 // substitution (zero carry from above) to the carry uin from below,
 // K(j) = H(j) + g(j) K(j+1) within the chunk, K(last) = H(last).  The rows
 // keep H's place; the look-back products use H itself.
-std::vector<double> fused_k_row(const FusedRows& r) {
+std::vector<double> fused_k_row(const FusedRows& r, int ch = FUSED_CH) {
     const int nzp = (int)r.HH.size();
     std::vector<double> K(nzp, 0.0);
-    for (int j0 = 0; j0 < nzp; j0 += FUSED_CH) {
-        const int j1 = j0 + FUSED_CH;
+    for (int j0 = 0; j0 < nzp; j0 += ch) {
+        const int j1 = j0 + ch;
         K[j1 - 1] = r.HH[j1 - 1];
         for (int j = j1 - 2; j >= j0; --j) K[j] = r.HH[j] + r.gg[j] * K[j + 1];
     }
@@ -174,6 +174,128 @@ bool fused_lookback_ok(int nz, int bcx, int bcp) {
         if (fused_lookback(fused_rows(nz, nzp, tri_for(nz, b)), tp, nz, f, g) > FUSED_LOOKBACK_BOUND) return false;
     }
     return true;
+}
+
+// Largest product of chunk multipliers that a carry of pencil.cu leaves out:
+// its scan reaches 16 chunks at least.
+double pencil_omitted(const FusedRows& r, int ch, int nz) {
+    const int nc = (nz + ch - 1) / ch;
+    double worst = 0.0;
+    for (int t = 0; t < nc; ++t) {
+        double pf = 1.0, pb = 1.0;
+        for (int i = 1; i <= 16; ++i) {
+            pf = (t - i >= 0) ? pf * r.HH[(size_t)(t - i) * ch + ch - 1] : 0.0;
+            pb = (t + i < nc) ? pb * r.GG[(size_t)(t + i) * ch] : 0.0;
+        }
+        worst = std::max(worst, std::max(std::fabs(pf), std::fabs(pb)));
+    }
+    return worst;
+}
+
+// Whether the carries of pencil.cu are exact to 2^-60 for the two boundary codes of a form
+bool pencil_ok(int nz, const PencilShape& sh, int bc1, int bc2) {
+    const int nzp = 32 * sh.W * sh.ch;
+    for (int b : {bc1, bc2})
+        if (pencil_omitted(fused_rows(nz, nzp, tri_for(nz, b), sh.ch), sh.ch, nz) > 8.6736173798840355e-19) return false;
+    return true;
+}
+
+// Values of the table of pencil.cu
+size_t pencil_table_size(const PencilShape& sh, int nzpml) {
+    const size_t tp = 32 * sh.W;
+    return PZ_COUNT * tp * sh.ch + 2 * PC_COUNT * tp + 4 * PE_COUNT + 3 * (size_t)nzpml;
+}
+
+// The table of pencil.cu (its order: internal.cuh)
+std::vector<double> pencil_table(int nz, int nb, int nt, const PencilShape& sh, int option, const double* zt,
+                                 const Tri* tri, const Compact<double>& cc) {
+    const int ch = sh.ch, tp = 32 * sh.W, nzp = tp * ch, nzpml = nb + nt;
+    std::vector<double> tab(pencil_table_size(sh, nzpml), 0.0);
+    auto put = [&](int row, int j, double v) { tab[(size_t)row * nzp + (size_t)(j % ch) * tp + j / ch] = v; };
+    auto Z = [&](int row, int j) { return zt[(size_t)row * nz + j]; };
+    for (int j = 0; j < nz; ++j) {
+        const double ri = Z(ZT_RHOINV, j), g = Z(ZT_G, j);
+        put(PZ_C2R, j, Z(ZT_C2RHO0, j));
+        put(PZ_GP, j, Z(ZT_GRADP0, j));
+        put(PZ_RI, j, ri);
+        put(PZ_E1, j, option == 2 ? g * ri : g * ri * Z(ZT_RHO0, j));
+        put(PZ_E2, j, g * ri * Z(ZT_GRADRHO0, j));
+        put(PZ_GR, j, Z(ZT_GRADRHO0, j));
+        put(PZ_R0, j, Z(ZT_RHO0, j));
+        put(PZ_SRC, j, Z(ZT_SRCDEP, j));
+    }
+    const double alpha = (double)(1.0f / 3.0f), ca = cc.C2 / alpha;     // the off-diagonal of tri_for
+    double* ce = tab.data() + (size_t)PZ_COUNT * nzp + (size_t)2 * PC_COUNT * tp;
+    const int bcs[2] = {option == 17 ? 3 : 1, option == 17 ? 2 : 0};
+    for (int k = 0; k < 2; ++k) {
+        const int bc = bcs[k];
+        const Tri& tr = tri[bc];
+        std::vector<double> sig(nzp, 1.0);
+        for (int j = 0; j < nz; ++j) sig[j] = Z(ZT_STRETCH, j) * (k == 1 ? Z(ZT_RHOINV, j) : 1.0);
+        const FusedRows r = fused_rows_scaled(fused_rows(nz, nzp, tr, ch), sig, ch);
+        const std::vector<double> kk = fused_k_row(r, ch);
+        const int base = k == 0 ? PZ_S1 : PZ_S2;
+        for (int j = 0; j < nzp; ++j) {
+            put(base + PS_D, j, (cc.C1 - ca) * r.ibd[j]);
+            put(base + PS_M, j, r.mm[j]);
+            put(base + PS_K, j, kk[j]);
+            put(base + PS_G, j, r.gg[j]);
+            put(base + PS_GC, j, r.GG[j]);
+            put(base + PS_A, j, (j > 0 && j < nz - 1) ? ca * sig[j] : 0.0);   // d1 counts as 0 on the end rows
+        }
+        // closures for y = f' - ca d1, d1 = 0 on the end rows: R' = R - ca A d1
+        // over the five levels from the end inwards (b0..b4), times 1/betad
+        for (int e = 0; e < 2; ++e) {
+            double* c = ce + (size_t)(2 * k + e) * PE_COUNT;
+            const double sg = e == 0 ? 1.0 : -1.0;               // the top rows are the mirrored ones with the sign changed
+            const int jn = e == 0 ? 1 : nz - 2, je = e == 0 ? 0 : nz - 1;
+            double near[5], end[5] = {0, 0, 0, 0, 0};
+            for (int i = 0; i < 5; ++i) near[i] = sg * cc.Cb[i];
+            const bool closed = e == 0 ? (bc == 1 || bc == 3) : (bc == 1 || bc == 2);
+            if (closed)
+                for (int i = 0; i < 5; ++i)
+                    end[i] = (cc.alpha2 * sg * (i < 4 ? cc.Cf[i] : 0.0) - cc.beta1 * near[i]) * cc.cnst;
+            // d1 of the second row: sg (b2 - b0), of the third: sg (b3 - b1)
+            const double off = e == 0 ? tr.upp[1] : tr.low[nz - 2], off_end = e == 0 ? tr.upp[0] : tr.low[nz - 1];
+            near[2] -= ca * sg; near[0] += ca * sg;
+            near[3] -= ca * sg * off; near[1] += ca * sg * off;
+            end[2] -= ca * sg * off_end; end[0] += ca * sg * off_end;
+            for (int i = 0; i < 5; ++i) {
+                c[i] = near[i] * r.ibd[jn];
+                c[5 + i] = end[i] * r.ibd[je];
+            }
+            c[PE_TOP] = (e == 1 && bc == 3) ? r.ibd[je] : 0.0;
+        }
+        double* c = tab.data() + (size_t)PZ_COUNT * nzp + (size_t)k * PC_COUNT * tp;
+        auto Mc = [&](int t) { return r.HH[(size_t)t * ch + ch - 1]; };
+        auto Gc = [&](int t) { return r.GG[(size_t)t * ch]; };
+        for (int t = 0; t < tp; ++t) {
+            const int lane = t % 32, w0 = t - lane;
+            for (int q = 0; q < 4; ++q) {
+                const int d = 1 << q;
+                double f = lane >= d ? 1.0 : 0.0, b = lane + d <= 31 ? 1.0 : 0.0;
+                for (int i = 1; i <= d && lane >= d; ++i) f *= Mc(t - i);
+                for (int i = 1; i <= d && lane + d <= 31; ++i) b *= Gc(t + i);
+                c[(size_t)(PC_F + q) * tp + t] = f;
+                c[(size_t)(PC_B + q) * tp + t] = b;
+            }
+            double fw = 1.0, bw = 1.0;
+            for (int i = w0; i < t; ++i) fw *= Mc(i);
+            for (int i = t + 1; i < w0 + 32; ++i) bw *= Gc(i);
+            c[(size_t)PC_FL * tp + t] = Mc(t);
+            c[(size_t)PC_FW * tp + t] = fw;
+            c[(size_t)PC_BL * tp + t] = Gc(t);
+            c[(size_t)PC_BW * tp + t] = bw;
+        }
+    }
+    double* pz = ce + 4 * PE_COUNT;
+    for (int ip = 0; ip < nzpml; ++ip) {
+        const int j = ip < nb ? ip : nz - nt + (ip - nb);
+        pz[ip] = Z(ZT_AZ, j);
+        pz[nzpml + ip] = Z(ZT_AZ, j) / Z(ZT_RHOINV, j);      // a_z of psi_p: the scale of the p' solve undone
+        pz[2 * nzpml + ip] = Z(ZT_BZ, j);
+    }
+    return tab;
 }
 
 // ddz of one z-profile (dbyd2 + stretch), divisions as in mtridag.f90:100-107
@@ -366,6 +488,28 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
         c->zt64 = (double*)c->zt;
         c->pt64 = (double*)c->pt;
     }
+    // FP64 quiet forms and the FP32 velocity form: the whole-step kernel of
+    // pencil.cu, where a pencil fits its shared memory and its carries are
+    // exact; SPARC_STAGE_LANES and SPARC_FP32_PER_STAGE ask for the per-stage
+    // kernels (the tests compare the two).  FP32 options 4 and 17 on more than
+    // 320 levels stay on the per-stage kernels: on some grids (8x4x321) the
+    // scaled solves' FP32 error is up to three times theirs.
+    {
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
+        cudaGetLastError();
+        const int opt = p->option, bc1 = opt == 17 ? 3 : 1, bc2 = opt == 17 ? 2 : 0;
+        c->pencil = pencil_shape(c->nz, c->M);
+        c->use_pencil = (opt == 2 || (!c->f32 && (opt == 4 || opt == 17))) &&
+                        getenv(c->f32 ? "SPARC_FP32_PER_STAGE" : "SPARC_STAGE_LANES") == nullptr &&
+                        pencil_count(c->pencil, opt, c->nzpml, (int)cs, 1, c->nsm) > 0 &&
+                        pencil_ok(c->nz, c->pencil, bc1, bc2) &&
+                        (c->f32 ? pencil_prepare<float>(c->pencil, opt, c->nzpml)
+                                : pencil_prepare<double>(c->pencil, opt, c->nzpml));
+        if (c->use_pencil && (rc = dalloc(c, &c->ptab, pencil_table_size(c->pencil, c->nzpml) * es))) return bail(rc);
+        if ((c->use_pencil || c->use_fused) &&
+            (rc = dalloc(c, &c->src_plane, (size_t)FUSED_STEPS * c->S * c->M * cs))) return bail(rc);
+    }
     // twiddle tables: n FP64 values, then the same n values in FP32
     if ((rc = dalloc(c, (void**)&c->tw_x, (size_t)p->nx * 12))) return bail(rc);
     if ((rc = dalloc(c, (void**)&c->tw_y, (size_t)std::max(p->ny, 2) * 12))) return bail(rc);
@@ -379,10 +523,7 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     c->t0.assign(c->S, 0);
     c->active_n = c->S;
     c->use_graphs = getenv("SPARC_NO_GRAPHS") == nullptr && !mhd_form;
-    if (c->use_fused) {
-        fused_prepare(c->nz, c->nzpml);
-        if ((rc = dalloc(c, &c->src_plane, (size_t)FUSED_STEPS * c->S * c->M * 8))) return bail(rc);
-    }
+    if (c->use_fused) fused_prepare(c->nz, c->nzpml);
     if (mhd_form && (rc = mhd_create(c))) return bail(rc);
     // twiddles cos/sin(2 pi q / n), q < n/2, exact pi; the FP32 copy (rounded
     // from FP64) follows the FP64 table in the same allocation
@@ -601,6 +742,16 @@ int sparc_gpu_set_background(sparc_ctx* c, const double* zin, const double* cin,
         }
     }
     int rc;
+    if (c->use_pencil) {
+        const std::vector<double> tab = pencil_table(nz, P.npmlbot, P.npmltop, c->pencil, P.option, c->zt_host.data(), tri, c->cc64);
+        if (c->f32) {
+            const std::vector<float> tf(tab.begin(), tab.end());
+            if ((rc = upload(c, c->ptab, tf.data(), tf.size() * 4))) return rc;
+        } else if ((rc = upload(c, c->ptab, tab.data(), tab.size() * 8))) {
+            return rc;
+        }
+        CK(cudaStreamSynchronize(c->stream));     // the host table goes out of scope
+    }
     if (c->f32) {
         if (c->use_fused) {
             // z table of the fused FP32 step, built in FP64 and rounded once:
@@ -1010,11 +1161,50 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
             Fz.nsteps = std::min(nsteps - it, FUSED_STEPS);
             Fz.write_scr = (it + Fz.nsteps == nsteps && c->rhs_out) ? 1 : 0;
             if (Fz.src_mode == 2) {
-                launch_source_plane(Fz, c->active_n, c->stream);
+                launch_source_plane<float>(Fz.src_plane, Fz.planes, Fz.plane_ss, Fz.L, Fz.clk, c->M, Fz.nsteps,
+                                           c->active_n, c->stream);
                 c->launches += 1;
             }
             launch_fused(Fz, c->active_n, c->stream);
             launch_tick(c->d_time, Fz.nsteps, c->stream);
+            c->launches += 2;
+            CKL();
+        }
+        return SPARC_OK;
+    }
+    if (c->use_pencil) {
+        PencilArgs<T> B;
+        memset(&B, 0, sizeof(B));
+        B.a = A.a; B.scr = A.scr; B.pml = A.pml;
+        B.tab = (const T*)c->ptab; B.pt = A.pt;
+        B.fs = A.fs; B.ps = A.ps; B.M = A.M; B.nz = A.nz; B.nzpml = c->nzpml;
+        B.npmlbot = A.npmlbot; B.npmltop = A.npmltop; B.option = A.option; B.damp = A.damp;
+        B.W = c->pencil.W;
+        B.nsrc = c->active_n;
+        B.pencils = c->pencil_tuned ? c->pencil_tuned
+                                    : pencil_count(c->pencil, A.option, c->nzpml, (int)csz(c),
+                                                   (long long)c->M * c->active_n, c->nsm);
+        B.unstr_top = (T)c->zt_host[(size_t)ZT_UNSTRETCH * c->nz + c->nz - 1];
+        B.dt = U.dt;
+        for (int i = 0; i < 5; ++i) B.betas[i] = (T)c->betas[i];
+        B.src_mode = A.src_mode; B.ksrc = A.ksrc; B.src_scale = A.src_scale;
+        B.planes = A.planes; B.plane_ss = A.plane_ss; B.L = A.L;
+        B.series = A.series; B.nseries = A.nseries;
+        B.src_plane = CP<T>(c->src_plane);
+        if (c->rec_on) {
+            B.rec = CP<T>(c->rec); B.rec_steps = c->steps; B.rec_max = c->rec_max; B.rec_k = c->o_rad - 1;
+        }
+        B.clk = A.clk;
+        for (int it = 0; it < nsteps; it += B.nsteps) {
+            B.nsteps = std::min(nsteps - it, FUSED_STEPS);
+            B.write_scr = (it + B.nsteps == nsteps && c->rhs_out) ? 1 : 0;
+            if (B.src_mode == 2) {
+                launch_source_plane<T>(B.src_plane, B.planes, B.plane_ss, B.L, B.clk, c->M, B.nsteps, c->active_n,
+                                       c->stream);
+                c->launches += 1;
+            }
+            launch_pencil<T>(B, c->pencil.ch, c->stream);
+            launch_tick(c->d_time, B.nsteps, c->stream);
             c->launches += 2;
             CKL();
         }
@@ -1138,6 +1328,19 @@ int sparc_gpu_set_mhd_background(sparc_ctx* c, const double* rho, const double* 
     return mhd_set_background(c, rho, cs, p, bx, by, bz);
 }
 
+// A launch variant of the autotuner: modes per CTA of the fused step, threads
+// per CTA of the other step kernels (the pencils that fill them in pencil.cu)
+static void set_variant(sparc_ctx* c, int v) {
+    if (c->use_fused && c->f32) {
+        c->fused_pencils = v;
+        return;
+    }
+    c->stage_block = v;
+    if (c->use_pencil)
+        c->pencil_tuned = std::min(std::max(1, v / (32 * c->pencil.W)),
+                                   pencil_count(c->pencil, c->P.option, c->nzpml, (int)csz(c), 1LL << 40, c->nsm));
+}
+
 int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step) {
     if (!c) return SPARC_EINVAL;
     if (!c->have_bg) return fail(c, SPARC_ESTATE, "set_background first");
@@ -1153,7 +1356,7 @@ int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step)
     int pick = cand[0];
     for (int ic = 0; ic < ncand; ++ic) {
         const int v = cand[ic];
-        if (fused) c->fused_pencils = v; else c->stage_block = v;
+        set_variant(c, v);
         c->epoch++;
         int rc = c->f32 ? do_steps<float>(c, steps) : do_steps<double>(c, steps);   // capture and warm
         if (!rc) {
@@ -1168,7 +1371,7 @@ int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step)
         ms /= steps;
         if (v == cand[0] || ms < best) { best = ms; pick = v; }
     }
-    if (fused) c->fused_pencils = pick; else c->stage_block = pick;
+    set_variant(c, pick);
     c->epoch++;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

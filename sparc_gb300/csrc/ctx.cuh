@@ -41,6 +41,11 @@ struct sparc_ctx {
     float* ftab = nullptr;                        // fused FP32 step: z table [FZ_COUNT][fused_nzp(nz)]
     int use_fused = 0;
     int fused_pencils = 4;                        // modes per CTA of the fused step (autotuned)
+    int use_pencil = 0;                           // whole-step kernel of pencil.cu
+    PencilShape pencil = {5, 1};
+    int pencil_tuned = 0;                         // pencils per CTA picked by the autotuner (0: by rule)
+    void* ptab = nullptr;                         // its T table
+    int nsm = 152;                                // SMs of the device
     int fused_test_nocopy = 0;                    // test switch: the fused step's table copy is not issued
     int stage_block = 128;                        // threads per CTA of the per-stage kernels (autotuned)
     int stage_q = 1, stage_chunk = 0;             // FP64 stage: lanes per pencil and levels per lane
@@ -54,7 +59,7 @@ struct sparc_ctx {
     double2* spec64b = nullptr;
     double2* tmp64 = nullptr;
     int* d_flag = nullptr;
-    void* src_plane = nullptr;    // [S][M] float2: the fused step's interpolated source plane
+    void* src_plane = nullptr;    // [FUSED_STEPS][S][M] CT: interpolated source planes of a launch's steps
     int rhs_out = 1;              // the last step of each step call leaves its right-hand side in scr
 
     // sources

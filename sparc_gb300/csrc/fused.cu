@@ -688,40 +688,48 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
     }
 }
 
-// LAGRANGE_INTERP source of the fused step (physics.f90:683-734): the plane
-// of every slot interpolated to the step about to run, sum over l of
+// LAGRANGE_INTERP source of the whole-step kernels (physics.f90:683-734): the
+// plane of every slot interpolated to the step about to run, sum over l of
 // w(l) * vr(l) with the FP64 weights of the slot's clock (samples that take
-// no part have weight 0 and are skipped), in FP32 in the order of l.  One
-// launch before each fused launch, for all its steps (grid.z), so that the
-// step's CTAs read one value instead of each computing the seven FP64 weights
-// on its critical path.
-__global__ void __launch_bounds__(256) source_plane_kernel(const FusedArgs A) {
+// no part have weight 0 and are skipped), in the order of l.  One launch
+// before each step launch, for all its steps (grid.z), so that the step's
+// CTAs read one value instead of each computing the seven FP64 weights on its
+// critical path.
+template <typename T>
+__global__ void __launch_bounds__(256) source_plane_kernel(typename CplxOf<T>::type* out,
+                                                           const typename CplxOf<T>::type* planes, long long plane_ss,
+                                                           int L, const SlotClock clk, int M, int nsrc) {
+    typedef typename CplxOf<T>::type CT;
     __shared__ double w[8];
     __shared__ int id[8];
     const int s = blockIdx.y;
     if (threadIdx.x < 7) {
-        const int tl = *A.clk.time - A.clk.t0[s] + (int)blockIdx.z;
+        const int tl = *clk.time - clk.t0[s] + (int)blockIdx.z;
         int i;
-        const double v = lagrange_weight(A.clk, tl, A.L, threadIdx.x, &i);
+        const double v = lagrange_weight(clk, tl, L, threadIdx.x, &i);
         w[threadIdx.x] = v;
         id[threadIdx.x] = i < 0 ? 0 : i;
     }
     __syncthreads();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= A.M) return;
-    const float2* pl = A.planes + (long long)s * A.plane_ss + m;
-    float2 F = make_float2(0.f, 0.f);
+    if (m >= M) return;
+    const CT* pl = planes + (long long)s * plane_ss + m;
+    CT F = czero<CT>();
     #pragma unroll
     for (int l = 0; l < 7; ++l)
-        if (w[l] != 0.0) F = F + (float)w[l] * pl[(long long)id[l] * A.M];
-    A.src_plane[((long long)blockIdx.z * A.nsrc + s) * A.M + m] = F;
+        if (w[l] != 0.0) F = F + (T)w[l] * pl[(long long)id[l] * M];
+    out[((long long)blockIdx.z * nsrc + s) * M + m] = F;
 }
 
-void launch_source_plane(const FusedArgs& A, int nsrc, cudaStream_t s) {
-    FusedArgs B = A;
-    B.nsrc = nsrc;
-    source_plane_kernel<<<dim3((A.M + 255) / 256, nsrc, A.nsteps), 256, 0, s>>>(B);
+template <typename T>
+void launch_source_plane(typename CplxOf<T>::type* out, const typename CplxOf<T>::type* planes, long long plane_ss,
+                         int L, const SlotClock& clk, int M, int nsteps, int nsrc, cudaStream_t s) {
+    source_plane_kernel<T><<<dim3((M + 255) / 256, nsrc, nsteps), 256, 0, s>>>(out, planes, plane_ss, L, clk, M, nsrc);
 }
+template void launch_source_plane<float>(float2*, const float2*, long long, int, const SlotClock&, int, int, int,
+                                         cudaStream_t);
+template void launch_source_plane<double>(double2*, const double2*, long long, int, const SlotClock&, int, int, int,
+                                          cudaStream_t);
 
 int fused_w(int nz) { return (nz + 32 * CH - 1) / (32 * CH); }
 int fused_nzp(int nz) { return 32 * CH * fused_w(nz); }

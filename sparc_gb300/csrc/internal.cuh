@@ -398,7 +398,62 @@ int fused_supported(int nz);
 int fused_w(int nz);
 int fused_nzp(int nz);
 void launch_fused(const FusedArgs& A, int nsrc, cudaStream_t s);
-void launch_source_plane(const FusedArgs& A, int nsrc, cudaStream_t s);
+
+// whole-step kernel on pencils (pencil.cu).  Table [PZ_COUNT][NZP], level
+// j = t CH + q of a row at q TP + t (consecutive threads read consecutive
+// values), then the carry rows [2][PC_COUNT][TP] and the closures
+// [2][2 ends][PE_COUNT] of the two solves, then a_z, a_z rho0 and b_z of the
+// PML planes.
+enum {      // elimination rows of a solve for the scaled unknown y
+    PS_D = 0,   // (C1 - C2 / alpha) / betad, the right-hand side's factor
+    PS_M,       // elimination multiplier
+    PS_K,       // response of the back-substituted chunk to the carry from below
+    PS_G,       // back-substitution multiplier
+    PS_GC,      // its products from the chunk's last level: response to the carry from above
+    PS_A,       // C2 / alpha, the part of f' outside y
+    PS_COUNT
+};
+enum {
+    PZ_C2R = 0, PZ_GP, PZ_RI, PZ_E1, PZ_E2, PZ_GR, PZ_R0, PZ_SRC,
+    PZ_S1, PZ_S2 = PZ_S1 + PS_COUNT, PZ_COUNT = PZ_S2 + PS_COUNT
+};
+enum {      // carry rows: products of chunk multipliers
+    PC_F = 0,           // over the 1, 2, 4, 8 chunks below, where the scan step stays in the warp
+    PC_FL = 4,          // of this chunk (the last lane's value for the next warp)
+    PC_FW,              // from the warp's first chunk to the one below this
+    PC_B,               // as PC_F from above
+    PC_BL = PC_B + 4, PC_BW, PC_COUNT
+};
+// closure coefficients of one end: the second row from the end (five), the
+// end row (five), and the factor of a caller-set end value
+enum { PE_TOP = 10, PE_COUNT = 12 };
+struct PencilShape { int ch, W; };      // levels per thread, warps per pencil
+template <typename T> struct PencilArgs {
+    typedef typename CplxOf<T>::type CT;
+    CT* a; CT* scr; CT* pml;
+    const T* tab; const T* pt;
+    long long fs, ps;
+    int M, nz, nzpml, npmlbot, npmltop, option, damp, W;
+    int pencils, nsrc, nsteps, write_scr;
+    T unstr_top, dt;
+    T betas[5];
+    int src_mode, ksrc;
+    T src_scale;
+    const CT* planes; long long plane_ss; int L;
+    const double* series; int nseries;
+    CT* src_plane;      // [nsteps][nsrc][M] each step's interpolated source plane (src_mode 2)
+    CT* rec;            // surface records, as FusedArgs
+    int rec_steps, rec_max, rec_k;
+    SlotClock clk;
+};
+PencilShape pencil_shape(int nz, int modes);
+int pencil_count(const PencilShape& sh, int option, int nzpml, int complex_bytes, long long pencils, int nsm);
+template <typename T> int pencil_prepare(const PencilShape& sh, int option, int nzpml);
+template <typename T> void launch_pencil(const PencilArgs<T>& A, int ch, cudaStream_t s);
+// each step's source plane of a launch of nsteps steps (fused.cu), LAGRANGE_INTERP
+template <typename T>
+void launch_source_plane(typename CplxOf<T>::type* out, const typename CplxOf<T>::type* planes, long long plane_ss,
+                         int L, const SlotClock& clk, int M, int nsteps, int nsrc, cudaStream_t s);
 
 // launchers (modal.cu)
 template <typename T> void launch_stage(const StageArgs<T>& A, int nsrc, cudaStream_t s);

@@ -36,10 +36,13 @@ def _all(s):
 
 
 @pytest.mark.parametrize("n", [2, 15, 16, 17, 33])
-@pytest.mark.parametrize("form,prec,lagrange", [("3d", "f32", False), ("3d", "f32", True), ("2d", "f32", True)])
+@pytest.mark.parametrize("form,prec,lagrange", [("3d", "f32", False), ("3d", "f32", True), ("2d", "f32", True),
+                                                ("3d", "f64", False), ("2d", "f64", True), ("vel", "f64", False),
+                                                ("vel", "f32", True)])
 def test_steps_of_one_call_equal_single_steps(gpu_lib, n, form, prec, lagrange):
     mk = small_params_2d if form == "2d" else small_params
-    p = mk(precision=prec, nsrc=3, compute_forward=not lagrange, compute_adjoint=lagrange)
+    kw = {"option": 2} if form == "vel" else {}
+    p = mk(precision=prec, nsrc=3, **kw, compute_forward=not lagrange, compute_adjoint=lagrange)
     with _build(p, lagrange) as one, _build(p, lagrange) as many:
         for s in (one, many):
             s.step(3)
@@ -49,3 +52,58 @@ def test_steps_of_one_call_equal_single_steps(gpu_lib, n, form, prec, lagrange):
         many.step(n)
         for x, y in zip(_all(one), _all(many)):
             assert np.array_equal(x, y)
+
+
+@pytest.fixture(scope="module")
+def oracle_mod():
+    from oracle import oracle
+    oracle.build()
+    return oracle
+
+
+# levels at the edges of the chunks (3 and 5 levels a thread) and of the warps
+# (96 and 160 levels), the smallest and the largest box, and both chunk rules:
+# 4 x 4 and 32 x 1 modes are few (3 levels a thread), 64 x 64 many
+@pytest.mark.parametrize("option,nx,ny,nz,nsteps", [
+    (4, 4, 4, 16, 31), (4, 8, 4, 96, 3), (4, 8, 8, 97, 3), (4, 4, 8, 193, 2), (4, 64, 64, 150, 2), (4, 64, 64, 160, 2),
+    (4, 64, 64, 161, 2), (4, 64, 64, 200, 2), (4, 8, 4, 321, 2), (4, 64, 64, 400, 1), (4, 4, 4, 1024, 1),
+    (17, 64, 1, 16, 31), (17, 64, 1, 95, 3), (17, 128, 1, 300, 31), (17, 8, 1, 769, 2),
+    (2, 4, 4, 17, 31), (2, 8, 4, 101, 3), (2, 64, 64, 101, 2), (2, 64, 64, 321, 1)])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_pencil_step_matches_oracle(gpu_lib, oracle_mod, option, nx, ny, nz, nsteps, prec):
+    """The whole-step kernel on chunked pencils (FP64, and FP32 in the velocity
+    form) against the FP64 oracle: FP64 <= 1e-10 relative L2 of the state and
+    the PML auxiliaries, FP32 <= 2e-5 of the state, as the other step kernels."""
+    if prec == "f32" and option != 2:
+        pytest.skip("FP32 options 4 and 17 do not run this kernel")
+    from cases import smooth_state
+    from sparc_gb300.background import polytrope_table
+    from sparc_gb300.solver import Solver
+    pml_n = max(2, min(10, nz // 6))
+    p = small_params(nx=nx, ny=ny, nz=nz, option=option, npmlbot=pml_n, npmltop=pml_n, precision=prec,
+                     src_k=nz // 2)
+    tab = polytrope_table(nz, z_bot_mm=-25.0 if nz > 100 else -6.0, z_top_mm=1.0)
+    a0, pml0 = smooth_state(p, seed=5)
+    if option == 2:
+        a0[5] = 0.0
+    plane = gaussian_plane(p)
+    series = oracle_mod.forward_source(p, 64) * 1e3
+    o = oracle_mod.Oracle(p, tab)
+    with Solver(p, tab) as g:
+        for s in (g, o):
+            s.set_state(a0, pml0)
+        g.set_source_series(plane, series)
+        # the oracle's delta_width is that of its default plane whatever src_k says
+        width = g.info()["delta_width"] / o.info()["delta_width"] if option != 2 else 1.0
+        o.set_source(1, plane[None] * width, series)
+        g.step(nsteps)
+        o.step(nsteps)
+        ag, pg = g.state()
+        rhs = np.stack([g.field(6 + f) for f in range(6)])
+    ao, so, po = o.state()
+    nrm = np.linalg.norm
+    tol = 1e-10 if prec == "f64" else 2e-5
+    assert nrm(ag - ao) <= tol * nrm(ao)
+    assert nrm(rhs - so) <= (1e-10 if prec == "f64" else 1e-3) * nrm(so)
+    if prec == "f64":
+        assert nrm(pg - po) <= tol * nrm(po)
