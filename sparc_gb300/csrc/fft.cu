@@ -1,7 +1,8 @@
 // Horizontal transforms between physical planes a(nx,ny) and the normalised
-// r2c half-spectrum state, written as shared-memory Stockham radix-2 FFTs
-// (the FFTW plans of initialize.f90:323-337 and damping.f90:46-58 are the
-// reference's counterpart; cuFFT is not used).
+// r2c half-spectrum state (the FFTW plans of initialize.f90:323-337 and
+// damping.f90:46-58 are the reference's counterpart; cuFFT is not used): the
+// register transforms of lines.cuh for 16 to 1024 points, shared-memory
+// Stockham radix-2 FFTs for 4 and 8.
 //
 //   phys -> spec : rows_r2c   (two real rows packed as one complex FFT along x,
 //                              split by Hermitian symmetry, scaled 1/(nx*ny))
@@ -12,13 +13,7 @@
 // Also: point-wise spectral multipliers and the sensitivity-kernel
 // accumulation of kernels.f90:273-311 on physical fields.
 #include "internal.cuh"
-
-// offset of input plane p when planes come in groups of ppg, group g starting
-// at g * gstride (complex elements); pe = elements per plane
-__device__ __forceinline__ long long grp_off(long long p, int ppg, long long gstride, long long pe) {
-    const long long g = p / ppg;
-    return g * gstride + (p - g * ppg) * pe;
-}
+#include "lines.cuh"
 
 // phys (nrows rows of nx reals) -> out (nrows rows of H = nx/2+1 complex), scaled by `scale`
 template <typename T>
@@ -117,242 +112,7 @@ __global__ void cols_fft_kernel(const typename CplxOf<T>::type* __restrict__ in,
     }
 }
 
-// ---- two-pass transforms for n = R*R (R = 8, 16): n = R*n1 + n2,
-// k = k1 + R*k2.  Pass 1 (thread n2): R-point DFT over n1 of x[R n1 + n2],
-// times the twiddle W_n^(n2 k1); pass 2 (thread k1): R-point DFT over n2.
-// Each DFT runs in registers; one shared-memory exchange and one barrier per
-// CTA.  W_m^j = exp(sign 2 pi i j / m) comes from the FP64 table tw
-// (cos, sin of 2 pi q / n for q < n/2).
-
-// complex FFT along y (length ny = R*R) for NC = 256/R kx-columns per CTA;
-// data [plane][y][kx] with H columns per row
-template <typename T, int R>
-__global__ void __launch_bounds__(256) cols_fft_sq_kernel(const typename CplxOf<T>::type* __restrict__ in,
-                                                          typename CplxOf<T>::type* __restrict__ out, int H,
-                                                          T sign, const double* __restrict__ tw, int ppg,
-                                                          long long gstride, const T* __restrict__ mul) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int n = R * R, NC = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    CT* Z = (CT*)smraw;                                  // [k1][n2][c]
-    const int ntile = (H + NC - 1) / NC;
-    const long long plane = blockIdx.x / ntile;
-    const int kx0 = (blockIdx.x % ntile) * NC;
-    const int c = threadIdx.x % NC, r = threadIdx.x / NC;
-    const bool cv = kx0 + c < H;
-    const long long base = plane * (long long)n * H + kx0 + c;
-    const long long ibase = grp_off(plane, ppg, gstride, (long long)n * H) + kx0 + c;
-    CT w[R / 2];
-    #pragma unroll
-    for (int j = 0; j < R / 2; ++j) w[j] = tw_n<T, CT>(tw, j * R, n, sign);
-    // pass 1: thread n2 = r
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) v[n1] = cv ? in[ibase + (long long)(R * n1 + r) * H] : czero<CT>();
-    reg_dft<CT, R>(v, w);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = v[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, n, sign));
-        Z[(k1 * R + r) * NC + c] = y;
-    }
-    __syncthreads();
-    // pass 2: thread k1 = r
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) v[n2] = Z[(r * R + n2) * NC + c];
-    reg_dft<CT, R>(v, w);
-    if (cv) {
-        #pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) {
-            CT val = v[brev<R>(k2)];
-            if (mul) val = __ldg(&mul[(long long)(r + R * k2) * H + kx0 + c]) * val;   // a real pencil multiplier
-            out[base + (long long)(r + R * k2) * H] = val;
-        }
-    }
-}
-
-// cols_fft_sq_kernel forward, the real multiplier mul[ky][kx], and
-// cols_fft_sq_kernel inverse in one pass, in place on [plane][y][kx] columns:
-// after the forward passes thread r holds the indices r + R k2, which are the
-// ones the inverse's first pass loads, so both halves are the standalone
-// kernels' arithmetic and the result equals the two-kernel path bit for bit
-template <typename T, int R>
-__global__ void __launch_bounds__(256) cols_filter_sq_kernel(typename CplxOf<T>::type* __restrict__ data, int H,
-                                                             const double* __restrict__ tw,
-                                                             const T* __restrict__ mul) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int n = R * R, NC = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    CT* Z = (CT*)smraw;                                  // [k1][n2][c]
-    const int ntile = (H + NC - 1) / NC;
-    const long long plane = blockIdx.x / ntile;
-    const int kx0 = (blockIdx.x % ntile) * NC;
-    const int c = threadIdx.x % NC, r = threadIdx.x / NC;
-    const bool cv = kx0 + c < H;
-    const long long base = plane * (long long)n * H + kx0 + c;
-    CT wf[R / 2], wi[R / 2];
-    #pragma unroll
-    for (int j = 0; j < R / 2; ++j) {
-        wf[j] = tw_n<T, CT>(tw, j * R, n, (T)-1);
-        wi[j] = tw_n<T, CT>(tw, j * R, n, (T)1);
-    }
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) v[n1] = cv ? data[base + (long long)(R * n1 + r) * H] : czero<CT>();
-    // forward, pass 1 (thread n2 = r) and pass 2 (thread k1 = r)
-    reg_dft<CT, R>(v, wf);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = v[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, n, (T)-1));
-        Z[(k1 * R + r) * NC + c] = y;
-    }
-    __syncthreads();
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) v[n2] = Z[(r * R + n2) * NC + c];
-    reg_dft<CT, R>(v, wf);
-    CT u[R];
-    #pragma unroll
-    for (int k2 = 0; k2 < R; ++k2) {
-        const CT X = v[brev<R>(k2)];
-        u[k2] = cv ? __ldg(&mul[(long long)(r + R * k2) * H + kx0 + c]) * X : czero<CT>();
-    }
-    __syncthreads();                                     // every thread has read its forward tile
-    // inverse, pass 1 (thread n2 = r holds indices R n1 + r) and pass 2
-    reg_dft<CT, R>(u, wi);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = u[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, n, (T)1));
-        Z[(k1 * R + r) * NC + c] = y;
-    }
-    __syncthreads();
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) u[n2] = Z[(r * R + n2) * NC + c];
-    reg_dft<CT, R>(u, wi);
-    if (cv) {
-        #pragma unroll
-        for (int k2 = 0; k2 < R; ++k2) data[base + (long long)(r + R * k2) * H] = u[brev<R>(k2)];
-    }
-}
-
-// inverse real transform along x (length nx = R*R), two rows per complex
-// FFT as rows_c2r_kernel, NP = 256/R row pairs per CTA
-template <typename T, int R>
-__global__ void __launch_bounds__(256) rows_c2r_sq_kernel(const typename CplxOf<T>::type* __restrict__ in,
-                                                          T* __restrict__ phys, long long nrows,
-                                                          const double* __restrict__ tw, int ny, int ppg,
-                                                          long long gstride) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int nx = R * R, H = nx / 2 + 1, half = nx / 2, NP = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    CT* Z = (CT*)smraw;                                  // [pair][k1][R+1]
-    const int r = threadIdx.x % R, pp = threadIdx.x / R;
-    const long long r0 = 2LL * ((long long)blockIdx.x * NP + pp), r1 = r0 + 1;
-    const bool has0 = r0 < nrows, has1 = r1 < nrows;
-    const long long pe = (long long)ny * H;
-    const long long o0 = has0 ? grp_off(r0 / ny, ppg, gstride, pe) + (r0 % ny) * H : 0;
-    const long long o1 = has1 ? grp_off(r1 / ny, ppg, gstride, pe) + (r1 % ny) * H : 0;
-    CT w[R / 2];
-    #pragma unroll
-    for (int j = 0; j < R / 2; ++j) w[j] = tw_n<T, CT>(tw, j * R, nx, (T)1);
-    // pass 1: thread n2 = r gathers z[R n1 + n2] of the packed pair
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) {
-        const int idx = R * n1 + r;
-        const bool mirror = idx > half;
-        const int k = mirror ? nx - idx : idx;
-        const CT x1 = has0 ? in[o0 + k] : czero<CT>();
-        const CT x2 = has1 ? in[o1 + k] : czero<CT>();
-        CT z;
-        if (k == 0 || k == half) { z.x = x1.x; z.y = x2.x; }
-        else if (!mirror) { z.x = x1.x - x2.y; z.y = x1.y + x2.x; }
-        else { z.x = x1.x + x2.y; z.y = -x1.y + x2.x; }
-        v[n1] = z;
-    }
-    reg_dft<CT, R>(v, w);
-    CT* Zp = Z + pp * R * (R + 1);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = v[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, nx, (T)1));
-        Zp[k1 * (R + 1) + r] = y;
-    }
-    __syncthreads();
-    // pass 2: thread k1 = r
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) v[n2] = Zp[r * (R + 1) + n2];
-    reg_dft<CT, R>(v, w);
-    #pragma unroll
-    for (int k2 = 0; k2 < R; ++k2) {
-        const CT zz = v[brev<R>(k2)];
-        if (has0) phys[r0 * nx + r + R * k2] = zz.x;
-        if (has1) phys[r1 * nx + r + R * k2] = zz.y;
-    }
-}
-
-// forward real transform along x (length nx = R*R) of two rows packed as one
-// complex FFT, split by Hermitian symmetry and scaled as rows_r2c_kernel;
-// NP = 256/R row pairs per CTA
-template <typename T, int R>
-__global__ void __launch_bounds__(256) rows_r2c_sq_kernel(const T* __restrict__ phys,
-                                                          typename CplxOf<T>::type* __restrict__ out,
-                                                          long long nrows, T scale, const double* __restrict__ tw) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int nx = R * R, H = nx / 2 + 1, NP = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int r = threadIdx.x % R, pp = threadIdx.x / R;
-    CT* Zp = (CT*)smraw + pp * R * (R + 1);              // [k1][R+1], then the spectrum [k]
-    const long long r0 = 2LL * ((long long)blockIdx.x * NP + pp), r1 = r0 + 1;
-    const bool has0 = r0 < nrows, has1 = r1 < nrows;
-    CT w[R / 2];
-    #pragma unroll
-    for (int j = 0; j < R / 2; ++j) w[j] = tw_n<T, CT>(tw, j * R, nx, (T)-1);
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) {
-        v[n1].x = has0 ? phys[r0 * nx + R * n1 + r] : (T)0;
-        v[n1].y = has1 ? phys[r1 * nx + R * n1 + r] : (T)0;
-    }
-    reg_dft<CT, R>(v, w);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = v[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, nx, (T)-1));
-        Zp[k1 * (R + 1) + r] = y;
-    }
-    __syncthreads();
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) v[n2] = Zp[r * (R + 1) + n2];
-    reg_dft<CT, R>(v, w);
-    __syncthreads();                                     // the tile now takes the spectrum
-    #pragma unroll
-    for (int k2 = 0; k2 < R; ++k2) Zp[r + R * k2] = v[brev<R>(k2)];
-    __syncthreads();
-    const T hs = (T)0.5 * scale;
-    for (int k = r; k < H; k += R) {
-        const CT zk = Zp[k], zn = Zp[(nx - k) & (nx - 1)];
-        CT x1, x2;
-        x1.x = (zk.x + zn.x) * hs;
-        x1.y = (zk.y - zn.y) * hs;
-        x2.x = (zk.y + zn.y) * hs;
-        x2.y = -(zk.x - zn.x) * hs;
-        if (has0) out[r0 * H + k] = x1;
-        if (has1) out[r1 * H + k] = x2;
-    }
-}
-
-static int sq_radix(int n) { return n == 256 ? 16 : (n == 64 ? 8 : 0); }
-
-static int col_tile(int ny) { return ny >= 1024 ? 4 : (ny >= 512 ? 8 : 16); }
-
-template <typename T>
-static void set_smem(const void* fn, size_t bytes) {
-    static size_t done = 0;
-    (void)done;
-    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
+static int col_tile(int) { return 16; }    // sizes below the line transforms (4, 8)
 
 // spec[plane][m] *= mul[m] (a real pencil multiplier, m < M)
 template <typename T>
@@ -369,24 +129,12 @@ template <typename T>
 static void rows_forward(const T* phys, typename CplxOf<T>::type* dst, int nx, long long nrows, T scale,
                          const double* tw_x, cudaStream_t s) {
     typedef typename CplxOf<T>::type CT;
-    const int Rx = sq_radix(nx);
-    if (Rx) {
-        const long long rows_per_cta = 2LL * (256 / Rx);
-        const unsigned grid = (unsigned)((nrows + rows_per_cta - 1) / rows_per_cta);
-        const size_t smr = (size_t)(256 / Rx) * Rx * (Rx + 1) * sizeof(CT);
-        if (Rx == 16) {
-            set_smem<T>((const void*)rows_r2c_sq_kernel<T, 16>, smr);
-            rows_r2c_sq_kernel<T, 16><<<grid, 256, smr, s>>>(phys, dst, nrows, scale, tw_x);
-        } else {
-            set_smem<T>((const void*)rows_r2c_sq_kernel<T, 8>, smr);
-            rows_r2c_sq_kernel<T, 8><<<grid, 256, smr, s>>>(phys, dst, nrows, scale, tw_x);
-        }
-    } else {
-        size_t sm = 2 * (size_t)nx * sizeof(CT);
-        int thr = nx / 2 < 256 ? (nx / 2 < 32 ? 32 : nx / 2) : 256;
-        set_smem<T>((const void*)rows_r2c_kernel<T>, sm);
-        rows_r2c_kernel<T><<<(unsigned)((nrows + 1) / 2), thr, sm, s>>>(phys, dst, nx, nrows, scale, tw_x);
+    if (line_ok(nx)) {
+        line_r2c<T>({{phys}, {dst}, 1, 0, 0}, 1, nx, nrows, scale, tw_x, {}, s);
+        return;
     }
+    size_t sm = 2 * (size_t)nx * sizeof(CT);
+    rows_r2c_kernel<T><<<(unsigned)((nrows + 1) / 2), 32, sm, s>>>(phys, dst, nx, nrows, scale, tw_x);
 }
 
 template <typename T>
@@ -399,28 +147,18 @@ void fft_phys_to_spec(const T* phys, typename CplxOf<T>::type* spec, typename Cp
     CT* dst = (ny == 1) ? spec : tmp;
     const T scale = (T)(1.0 / ((double)nx * ny));
     rows_forward<T>(phys, dst, nx, nrows, scale, tw_x, s);
-    const int Ry = sq_radix(ny);
-    if (ny > 1 && Ry) {
-        const int NC = 256 / Ry, ntile = (H + NC - 1) / NC;
-        const size_t smc = (size_t)ny * NC * sizeof(CT);
-        if (Ry == 16) {
-            set_smem<T>((const void*)cols_fft_sq_kernel<T, 16>, smc);
-            cols_fft_sq_kernel<T, 16><<<(unsigned)(ntile * (long long)nplanes), 256, smc, s>>>(tmp, spec, H, (T)-1,
-                                                                                             tw_y, nplanes, 0LL, mul);
-        } else {
-            set_smem<T>((const void*)cols_fft_sq_kernel<T, 8>, smc);
-            cols_fft_sq_kernel<T, 8><<<(unsigned)(ntile * (long long)nplanes), 256, smc, s>>>(tmp, spec, H, (T)-1,
-                                                                                            tw_y, nplanes, 0LL, mul);
-        }
-    } else if (ny > 1) {
+    if (ny > 1 && line_ok(ny)) {
+        line_cols<T>(tmp, spec, H, ny, nplanes, nplanes, 0LL, -1, mul, tw_y, s);
+        return;
+    }
+    if (ny > 1) {
         int W = col_tile(ny);
         size_t sm2 = 2 * (size_t)W * ny * sizeof(CT);
-        set_smem<T>((const void*)cols_fft_kernel<T>, sm2);
         int ntile = (H + W - 1) / W;
         cols_fft_kernel<T><<<(unsigned)(ntile * (long long)nplanes), 256, sm2, s>>>(tmp, spec, ny, H, W, (T)-1, tw_y,
                                                                                    nplanes, 0LL);
     }
-    if (mul && !(ny > 1 && Ry)) {
+    if (mul) {
         const long long n = (long long)nplanes * ny * H;
         spec_mul_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(spec, mul, ny * H, n);
     }
@@ -431,24 +169,12 @@ template <typename T>
 static void rows_inverse(const typename CplxOf<T>::type* src, T* phys, int nx, int ny, long long nrows,
                          int rppg, long long rgs, const double* tw_x, cudaStream_t s) {
     typedef typename CplxOf<T>::type CT;
-    const int Rx = sq_radix(nx);
-    const long long npairs = (nrows + 1) / 2;
-    if (Rx == 16) {
-        const size_t sm = (size_t)16 * 16 * 17 * sizeof(CT);
-        set_smem<T>((const void*)rows_c2r_sq_kernel<T, 16>, sm);
-        rows_c2r_sq_kernel<T, 16><<<(unsigned)((npairs + 15) / 16), 256, sm, s>>>(src, phys, nrows, tw_x, ny, rppg, rgs);
-        return;
-    }
-    if (Rx == 8) {
-        const size_t sm = (size_t)32 * 8 * 9 * sizeof(CT);
-        set_smem<T>((const void*)rows_c2r_sq_kernel<T, 8>, sm);
-        rows_c2r_sq_kernel<T, 8><<<(unsigned)((npairs + 31) / 32), 256, sm, s>>>(src, phys, nrows, tw_x, ny, rppg, rgs);
+    if (line_ok(nx)) {
+        line_c2r<T>({{src}, {phys}, 1, 0, 0}, 1, nx, ny, nrows, rppg, rgs, tw_x, {}, s);
         return;
     }
     size_t sm = 2 * (size_t)nx * sizeof(CT);
-    int thr = nx / 2 < 256 ? (nx / 2 < 32 ? 32 : nx / 2) : 256;
-    set_smem<T>((const void*)rows_c2r_kernel<T>, sm);
-    rows_c2r_kernel<T><<<(unsigned)npairs, thr, sm, s>>>(src, phys, nx, nrows, tw_x, ny, rppg, rgs);
+    rows_c2r_kernel<T><<<(unsigned)((nrows + 1) / 2), 32, sm, s>>>(src, phys, nx, nrows, tw_x, ny, rppg, rgs);
 }
 
 template <typename T>
@@ -462,21 +188,11 @@ void fft_spec_to_phys_g(const typename CplxOf<T>::type* spec, int ppg, long long
     int rppg = ppg;
     long long rgs = gstride;
     if (ny > 1) {
-        const int Ry = sq_radix(ny);
-        const unsigned blocks16 = (unsigned)(((H + 15) / 16) * (long long)nplanes);
-        const unsigned blocks8 = (unsigned)(((H + 31) / 32) * (long long)nplanes);
-        if (Ry == 16) {
-            const size_t sm2 = (size_t)16 * 16 * 16 * sizeof(CT);
-            set_smem<T>((const void*)cols_fft_sq_kernel<T, 16>, sm2);
-            cols_fft_sq_kernel<T, 16><<<blocks16, 256, sm2, s>>>(spec, tmp, H, (T)1, tw_y, ppg, gstride, nullptr);
-        } else if (Ry == 8) {
-            const size_t sm2 = (size_t)8 * 8 * 32 * sizeof(CT);
-            set_smem<T>((const void*)cols_fft_sq_kernel<T, 8>, sm2);
-            cols_fft_sq_kernel<T, 8><<<blocks8, 256, sm2, s>>>(spec, tmp, H, (T)1, tw_y, ppg, gstride, nullptr);
+        if (line_ok(ny)) {
+            line_cols<T>(spec, tmp, H, ny, nplanes, ppg, gstride, 1, nullptr, tw_y, s);
         } else {
             int W = col_tile(ny);
             size_t sm2 = 2 * (size_t)W * ny * sizeof(CT);
-            set_smem<T>((const void*)cols_fft_kernel<T>, sm2);
             int ntile = (H + W - 1) / W;
             cols_fft_kernel<T><<<(unsigned)(ntile * (long long)nplanes), 256, sm2, s>>>(spec, tmp, ny, H, W, (T)1, tw_y,
                                                                                        ppg, gstride);
@@ -489,32 +205,21 @@ void fft_spec_to_phys_g(const typename CplxOf<T>::type* spec, int ppg, long long
 }
 
 // phys -> out through the half spectrum times the real pencil multiplier
-// mul[ky][kx] (damping, horizontal filter).  For ny = 64 or 256 the column
-// passes run as one kernel in place on tmp (3 launches); otherwise as
-// fft_phys_to_spec + fft_spec_to_phys through spec (4 or 5).  Returns the
-// number of launches.
+// mul[ky][kx] (damping, horizontal filter).  The column passes run as one
+// kernel in place on tmp (3 launches) where the line transforms cover ny;
+// otherwise as fft_phys_to_spec + fft_spec_to_phys through spec (3 to 5).
+// Returns the number of launches.
 template <typename T>
 int fft_filter_phys(const T* phys, T* out, typename CplxOf<T>::type* spec, typename CplxOf<T>::type* tmp, int nx,
                     int ny, int nplanes, const double* tw_x, const double* tw_y, cudaStream_t s, const T* mul) {
-    typedef typename CplxOf<T>::type CT;
-    const int Ry = sq_radix(ny);
-    if (!(ny > 1 && Ry)) {
+    if (!(ny > 1 && line_ok(ny))) {
         fft_phys_to_spec<T>(phys, spec, tmp, nx, ny, nplanes, tw_x, tw_y, s, mul);
         fft_spec_to_phys<T>(spec, out, tmp, nx, ny, nplanes, tw_x, tw_y, s);
         return ny > 1 ? 5 : 3;
     }
-    const int H = nx / 2 + 1;
     const long long nrows = (long long)ny * nplanes;
     rows_forward<T>(phys, tmp, nx, nrows, (T)(1.0 / ((double)nx * ny)), tw_x, s);
-    const int NC = 256 / Ry, ntile = (H + NC - 1) / NC;
-    const size_t smc = (size_t)ny * NC * sizeof(CT);
-    if (Ry == 16) {
-        set_smem<T>((const void*)cols_filter_sq_kernel<T, 16>, smc);
-        cols_filter_sq_kernel<T, 16><<<(unsigned)(ntile * (long long)nplanes), 256, smc, s>>>(tmp, H, tw_y, mul);
-    } else {
-        set_smem<T>((const void*)cols_filter_sq_kernel<T, 8>, smc);
-        cols_filter_sq_kernel<T, 8><<<(unsigned)(ntile * (long long)nplanes), 256, smc, s>>>(tmp, H, tw_y, mul);
-    }
+    line_cols_filter<T>({{tmp}, {tmp}, 1, 0, 0}, 1, nx / 2 + 1, ny, nplanes, mul, tw_y, {}, s);
     rows_inverse<T>(tmp, out, nx, ny, nrows, nplanes, 0LL, tw_x, s);
     return 3;
 }

@@ -199,7 +199,7 @@ __device__ __forceinline__ int lagrange_dev(const SlotClock& k, int tl, int L, i
     return n;
 }
 
-// ---- register DFTs of the two-pass transforms (n = R*R) -----------------------
+// ---- twiddles of the transforms -------------------------------------------------
 // W_n^q = exp(sign 2 pi i q / n) for 0 <= q < n from a table of n values
 // (cos, sin of 2 pi q / n for q < n/2) in FP64, followed by the same n values
 // in FP32 (read by the FP32 kernels, so no conversion on the FP64 pipe)
@@ -245,35 +245,6 @@ __device__ __forceinline__ float2 bdif(float2 a, float2 c) { return __ffma2_rn(m
 __device__ __forceinline__ float2 bsum(float2 a, float2 c) { return a + c; }
 __device__ __forceinline__ float2 bdif(float2 a, float2 c) { return make_float2(a.x - c.x, a.y - c.y); }
 #endif
-
-// in-register DFT of length R (decimation in frequency): on return v[brev(k)]
-// holds X[k]; w[j] = W_R^j for j < R/2
-template <typename CT, int R>
-__device__ __forceinline__ void reg_dft(CT (&v)[R], const CT (&w)[R / 2]) {
-    #pragma unroll
-    for (int len = R; len >= 2; len >>= 1) {
-        const int half = len >> 1, step = R / len;
-        #pragma unroll
-        for (int b = 0; b < R; b += len) {
-            #pragma unroll
-            for (int k = 0; k < half; ++k) {
-                const CT a = v[b + k], c = v[b + k + half];
-                v[b + k] = bsum(a, c);
-                const CT d = bdif(a, c);
-                v[b + k + half] = (k == 0) ? d : cmul(d, w[k * step]);
-            }
-        }
-    }
-}
-
-template <int R>
-__host__ __device__ constexpr int brev(int k) {
-    int r = 0;
-    for (int b = 1, m = R >> 1; b < R; b <<= 1, m >>= 1)
-        if (k & b) r |= m;
-    return r;
-}
-
 
 // Stockham radix-2 over `count` sequences of length n stored back to back in
 // src; returns the buffer that holds the result.  tw[2q], tw[2q+1] =

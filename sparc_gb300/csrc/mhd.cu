@@ -4,7 +4,7 @@
 // quiet-Sun path, so here the state lives in physical space: each
 // [source][field] slot of the context holds one dense (nz, ny, nx) real
 // field, and a stage takes its 21 derivatives explicitly:
-//   d/dx  two real rows packed as one complex row, shared-memory FFT, times
+//   d/dx  two real rows packed as one complex row, FFT (lines.cuh), times
 //         i k normx 2 pi stretchx (the reference's eyekx * stretchx, Nyquist
 //         dropped as its c2r does), inverse FFT  (derivatives.f90:28-58);
 //   d/dy  two adjacent x-columns packed as one complex column, the same
@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "ctx.cuh"
+#include "lines.cuh"
 
 namespace {
 
@@ -115,113 +116,6 @@ __global__ void rowderiv_kernel(const T* __restrict__ in, T* __restrict__ out, i
     for (int i = threadIdx.x; i < nx; i += blockDim.x) {
         out[r0 * nx + i] = Y[i].x;
         if (has1) out[r1 * nx + i] = Y[i].y;
-    }
-}
-
-// ---- spectral derivative of packed lines of length n = R*R (R = 8, 16) ------
-// Thread r holds v[n1] = z[R n1 + r] of one packed line z (two real lines as
-// real and imaginary parts).  Forward two-pass DFT (n = R n1 + n2, k = k1 +
-// R k2: thread n2 does the DFT over n1, twiddle W^(n2 k1), exchange, thread k1
-// the DFT over n2), times i*mul[k], then the inverse in the mirrored order
-// (thread k1: DFT over k2, twiddle W^-(n2 k1), exchange, thread n2: DFT over
-// k1), so that on return v[n1] holds the derivative at R n1 + r again.  The
-// derivative operator is real, so the two packed lines stay separate.
-// zs(a, b) is the exchange cell (row a, column b) of this line's R x R tile.
-template <typename T, typename CT, int R, typename ZS>
-__device__ __forceinline__ void deriv_sq(CT (&v)[R], int r, ZS zs, const T* __restrict__ mul,
-                                         const double* __restrict__ tw) {
-    constexpr int n = R * R;
-    CT wf[R / 2], wi[R / 2];
-    #pragma unroll
-    for (int j = 0; j < R / 2; ++j) {
-        wf[j] = tw_n<T, CT>(tw, j * R, n, (T)-1);
-        wi[j] = tw_n<T, CT>(tw, j * R, n, (T)1);
-    }
-    reg_dft<CT, R>(v, wf);
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) {
-        CT y = v[brev<R>(k1)];
-        if (k1 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * k1, n, (T)-1));
-        zs(k1, r) = y;
-    }
-    __syncthreads();
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) v[n2] = zs(r, n2);
-    __syncthreads();                                   // the tile is rewritten below
-    reg_dft<CT, R>(v, wf);
-    CT u[R];
-    #pragma unroll
-    for (int k2 = 0; k2 < R; ++k2) {
-        const CT X = v[brev<R>(k2)];
-        const T m = __ldg(&mul[r + R * k2]);
-        u[k2].x = -m * X.y;
-        u[k2].y = m * X.x;
-    }
-    reg_dft<CT, R>(u, wi);
-    #pragma unroll
-    for (int n2 = 0; n2 < R; ++n2) {
-        CT y = u[brev<R>(n2)];
-        if (n2 > 0 && r > 0) y = cmul(y, tw_n<T, CT>(tw, r * n2, n, (T)1));
-        zs(n2, r) = y;
-    }
-    __syncthreads();
-    #pragma unroll
-    for (int k1 = 0; k1 < R; ++k1) u[k1] = zs(r, k1);
-    reg_dft<CT, R>(u, wi);
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) v[n1] = u[brev<R>(n1)];
-}
-
-// d/dx of nrows dense rows of nx = R*R reals: 256/R row pairs per CTA, R
-// threads per pair
-template <typename T, int R>
-__global__ void __launch_bounds__(256) rowderiv_sq_kernel(const T* __restrict__ in, T* __restrict__ out,
-                                                          long long nrows, const T* __restrict__ mul,
-                                                          const double* __restrict__ tw) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int nx = R * R, NPR = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    const int r = threadIdx.x % R, pp = threadIdx.x / R;
-    CT* Zp = (CT*)smraw + pp * R * (R + 1);
-    const long long r0 = 2LL * ((long long)blockIdx.x * NPR + pp), r1 = r0 + 1;
-    const bool has0 = r0 < nrows, has1 = r1 < nrows;
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) {
-        v[n1].x = has0 ? in[r0 * nx + R * n1 + r] : (T)0;
-        v[n1].y = has1 ? in[r1 * nx + R * n1 + r] : (T)0;
-    }
-    deriv_sq<T, CT, R>(v, r, [&](int a, int b) -> CT& { return Zp[a * (R + 1) + b]; }, mul, tw);
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) {
-        if (has0) out[r0 * nx + R * n1 + r] = v[n1].x;
-        if (has1) out[r1 * nx + R * n1 + r] = v[n1].y;
-    }
-}
-
-// d/dy of nplanes dense (ny, nx) planes, ny = R*R: 256/R pairs of adjacent
-// x-columns per CTA (read and written as one complex value), R threads per pair
-template <typename T, int R>
-__global__ void __launch_bounds__(256) colderiv_sq_kernel(const T* __restrict__ in, T* __restrict__ out, int nx,
-                                                          const T* __restrict__ mul, const double* __restrict__ tw) {
-    typedef typename CplxOf<T>::type CT;
-    constexpr int ny = R * R, NC = 256 / R;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    CT* Z = (CT*)smraw;
-    const int npair = nx / 2, ntile = (npair + NC - 1) / NC;
-    const long long plane = blockIdx.x / ntile;
-    const int c = threadIdx.x % NC, r = threadIdx.x / NC;
-    const int cp = (blockIdx.x % ntile) * NC + c;
-    const bool cv = cp < npair;
-    const CT* src = (const CT*)(in + plane * (long long)ny * nx) + cp;
-    CT* dst = (CT*)(out + plane * (long long)ny * nx) + cp;
-    CT v[R];
-    #pragma unroll
-    for (int n1 = 0; n1 < R; ++n1) v[n1] = cv ? src[(long long)(R * n1 + r) * npair] : czero<CT>();
-    deriv_sq<T, CT, R>(v, r, [&](int a, int b) -> CT& { return Z[(a * R + b) * NC + c]; }, mul, tw);
-    if (cv) {
-        #pragma unroll
-        for (int n1 = 0; n1 < R; ++n1) dst[(long long)(R * n1 + r) * npair] = v[n1];
     }
 }
 
@@ -922,25 +816,14 @@ template <typename T>
 int ddx_launch(sparc_ctx* c, const T* in, T* out, long long nplanes) {
     const int nx = c->P.nx;
     const long long nrows = nplanes * c->P.ny;
-    typedef typename CplxOf<T>::type CT;
-    if (nx == 256 || nx == 64) {
-        const long long rows_per_cta = 2LL * (256 / (nx == 256 ? 16 : 8));
-        const unsigned grid = (unsigned)((nrows + rows_per_cta - 1) / rows_per_cta);
-        if (nx == 256) {
-            const size_t sm = (size_t)16 * 16 * 17 * sizeof(CT);
-            cudaFuncSetAttribute((const void*)rowderiv_sq_kernel<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            rowderiv_sq_kernel<T, 16><<<grid, 256, sm, c->stream>>>(in, out, nrows, (const T*)c->mhd->rx, c->tw_x);
-        } else {
-            const size_t sm = (size_t)32 * 8 * 9 * sizeof(CT);
-            rowderiv_sq_kernel<T, 8><<<grid, 256, sm, c->stream>>>(in, out, nrows, (const T*)c->mhd->rx, c->tw_x);
-        }
+    if (line_ok(nx)) {
+        line_rows<T>({{in}, {out}, 1, 0, 0}, 1, nx, nrows, (const T*)c->mhd->rx, false, c->tw_x, {}, c->stream);
         c->launches++;
         CKL();
         return SPARC_OK;
     }
     const size_t sm = 2 * (size_t)nx * sizeof(typename CplxOf<T>::type);
-    const int thr = nx / 2 < 32 ? 32 : (nx / 2 > 256 ? 256 : nx / 2);
-    rowderiv_kernel<T><<<(unsigned)((nrows + 1) / 2), thr, sm, c->stream>>>(in, out, nx, nrows, (const T*)c->mhd->rx,
+    rowderiv_kernel<T><<<(unsigned)((nrows + 1) / 2), 32, sm, c->stream>>>(in, out, nx, nrows, (const T*)c->mhd->rx,
                                                                            c->tw_x);
     c->launches++;
     CKL();
@@ -950,20 +833,8 @@ int ddx_launch(sparc_ctx* c, const T* in, T* out, long long nplanes) {
 template <typename T>
 int ddy_launch(sparc_ctx* c, const T* in, T* out, long long nplanes) {
     const int nx = c->P.nx, ny = c->P.ny;
-    typedef typename CplxOf<T>::type CT;
-    if (ny == 256 || ny == 64) {
-        const int R = ny == 256 ? 16 : 8, NC = 256 / R;
-        const long long ntile = (nx / 2 + NC - 1) / NC;
-        const size_t sm = (size_t)R * R * NC * sizeof(CT);
-        if (ny == 256) {
-            cudaFuncSetAttribute((const void*)colderiv_sq_kernel<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            colderiv_sq_kernel<T, 16><<<(unsigned)(nplanes * ntile), 256, sm, c->stream>>>(in, out, nx, (const T*)c->mhd->ry,
-                                                                                        c->tw_y);
-        } else {
-            cudaFuncSetAttribute((const void*)colderiv_sq_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            colderiv_sq_kernel<T, 8><<<(unsigned)(nplanes * ntile), 256, sm, c->stream>>>(in, out, nx, (const T*)c->mhd->ry,
-                                                                                       c->tw_y);
-        }
+    if (line_ok(ny)) {
+        line_cols_deriv<T>({{in}, {out}, 1, 0, 0}, 1, nx, ny, nplanes, (const T*)c->mhd->ry, c->tw_y, c->stream);
         c->launches++;
         CKL();
         return SPARC_OK;
