@@ -11,6 +11,7 @@
 #include <algorithm>
 
 #include "ctx.cuh"
+#include "zsolve.cuh"
 #include "adjsrc.cuh"
 #include "update.cuh"
 
@@ -140,11 +141,12 @@ std::vector<double> fused_k_row(const FusedRows& r, int ch = FUSED_CH) {
 // the largest product over FUSED_KB chunks, the factor of the first chunk the
 // carries leave out, over the chunks that hold real levels (the carries into
 // padding chunks reach no real row: their H and G rows are zero).
-double fused_lookback(const FusedRows& r, int tp, int nz, std::vector<double>& fwd, std::vector<double>& bwd) {
+double fused_lookback(const FusedRows& r, int tp, int nz, std::vector<double>& fwd, std::vector<double>& bwd,
+                      int ch = FUSED_CH) {
     std::vector<double> Mc(tp), Gc(tp);
     for (int t = 0; t < tp; ++t) {
-        Mc[t] = r.HH[t * FUSED_CH + FUSED_CH - 1];
-        Gc[t] = r.GG[t * FUSED_CH];
+        Mc[t] = r.HH[t * ch + ch - 1];
+        Gc[t] = r.GG[t * ch];
     }
     fwd.assign((size_t)4 * tp, 0.0);
     bwd.assign((size_t)4 * tp, 0.0);
@@ -157,7 +159,7 @@ double fused_lookback(const FusedRows& r, int tp, int nz, std::vector<double>& f
             if (i <= FUSED_KB) {
                 fwd[(size_t)4 * t + i - 2] = pf;
                 bwd[(size_t)4 * t + i - 2] = pb;
-            } else if (t * FUSED_CH < nz) {
+            } else if (t * ch < nz) {
                 worst = std::max(worst, std::max(std::fabs(pf), std::fabs(pb)));
             }
         }
@@ -200,6 +202,64 @@ bool pencil_ok(int nz, const PencilShape& sh, int bc1, int bc2) {
     return true;
 }
 
+// The scheme's solves for y = f' - (C2/alpha) d1, d1(j) = f(j+1) - f(j-1):
+// C2 / alpha, alpha the off-diagonal of tri_for
+double d1_factor(const Compact<double>& cc) { return cc.C2 / (double)(1.0f / 3.0f); }
+
+// Closure coefficients of one end (e = 0 bottom, 1 top; PE_* layout) for y, with
+// d1 = 0 on the end rows: R' = R - (C2/alpha) A d1 over the five levels from the
+// end inwards (b0..b4), times 1/betad
+void closure_row(double* c, int e, int nz, int bc, const Tri& tr, const std::vector<double>& ibd,
+                 const Compact<double>& cc) {
+    const double ca = d1_factor(cc), sg = e == 0 ? 1.0 : -1.0;   // the top rows are the mirrored ones with the sign changed
+    const int jn = e == 0 ? 1 : nz - 2, je = e == 0 ? 0 : nz - 1;
+    double near[5], end[5] = {0, 0, 0, 0, 0};
+    for (int i = 0; i < 5; ++i) near[i] = sg * cc.Cb[i];
+    const bool closed = e == 0 ? (bc == 1 || bc == 3) : (bc == 1 || bc == 2);
+    if (closed)
+        for (int i = 0; i < 5; ++i)
+            end[i] = (cc.alpha2 * sg * (i < 4 ? cc.Cf[i] : 0.0) - cc.beta1 * near[i]) * cc.cnst;
+    // d1 of the second row: sg (b2 - b0), of the third: sg (b3 - b1)
+    const double off = e == 0 ? tr.upp[1] : tr.low[nz - 2], off_end = e == 0 ? tr.upp[0] : tr.low[nz - 1];
+    near[2] -= ca * sg; near[0] += ca * sg;
+    near[3] -= ca * sg * off; near[1] += ca * sg * off;
+    end[2] -= ca * sg * off_end; end[0] += ca * sg * off_end;
+    for (int i = 0; i < 5; ++i) {
+        c[i] = near[i] * ibd[jn];
+        c[5 + i] = end[i] * ibd[je];
+    }
+    c[PE_TOP] = (e == 1 && bc == 3) ? ibd[je] : 0.0;
+}
+
+// The table of zsolve.cuh: d/dz times stretch, the four boundary codes
+std::vector<double> z_table(int nz, const std::vector<double>& stretch, const Tri* tri, const Compact<double>& cc) {
+    const int nw = z_chunks(nz), nzp = nw * ZCS, size = z_code_size(nz);
+    std::vector<double> tab((size_t)4 * size, 0.0), sig(nzp, 1.0);
+    std::copy(stretch.begin(), stretch.end(), sig.begin());
+    const double ca = d1_factor(cc);
+    for (int bc = 0; bc < 4; ++bc) {
+        double* t = tab.data() + (size_t)bc * size;
+        const FusedRows r = fused_rows_scaled(fused_rows(nz, nzp, tri[bc], ZCS), sig, ZCS);
+        const std::vector<double> kk = fused_k_row(r, ZCS);
+        for (int j = 0; j < nzp; ++j) {
+            t[PS_D * nzp + j] = (cc.C1 - ca) * r.ibd[j];
+            t[PS_M * nzp + j] = r.mm[j];
+            t[PS_K * nzp + j] = kk[j];
+            t[PS_G * nzp + j] = r.gg[j];
+            t[PS_GC * nzp + j] = r.GG[j];
+            t[PS_A * nzp + j] = (j > 0 && j < nz - 1) ? ca * sig[j] : 0.0;
+        }
+        std::vector<double> f, b;
+        fused_lookback(r, nw, nz, f, b, ZCS);
+        static_assert(ZKB == FUSED_KB, "fused_lookback's chunks");
+        std::copy(f.begin(), f.end(), t + PS_COUNT * nzp);
+        std::copy(b.begin(), b.end(), t + PS_COUNT * nzp + nw * (ZKB - 1));
+        for (int e = 0; e < 2; ++e)
+            closure_row(t + PS_COUNT * nzp + 2 * nw * (ZKB - 1) + e * PE_COUNT, e, nz, bc, tri[bc], r.ibd, cc);
+    }
+    return tab;
+}
+
 // Values of the table of pencil.cu
 size_t pencil_table_size(const PencilShape& sh, int nzpml) {
     const size_t tp = 32 * sh.W;
@@ -224,7 +284,7 @@ std::vector<double> pencil_table(int nz, int nb, int nt, const PencilShape& sh, 
         put(PZ_R0, j, Z(ZT_RHO0, j));
         put(PZ_SRC, j, Z(ZT_SRCDEP, j));
     }
-    const double alpha = (double)(1.0f / 3.0f), ca = cc.C2 / alpha;     // the off-diagonal of tri_for
+    const double ca = d1_factor(cc);
     double* ce = tab.data() + (size_t)PZ_COUNT * nzp + (size_t)2 * PC_COUNT * tp;
     const int bcs[2] = {option == 17 ? 3 : 1, option == 17 ? 2 : 0};
     for (int k = 0; k < 2; ++k) {
@@ -243,29 +303,7 @@ std::vector<double> pencil_table(int nz, int nb, int nt, const PencilShape& sh, 
             put(base + PS_GC, j, r.GG[j]);
             put(base + PS_A, j, (j > 0 && j < nz - 1) ? ca * sig[j] : 0.0);   // d1 counts as 0 on the end rows
         }
-        // closures for y = f' - ca d1, d1 = 0 on the end rows: R' = R - ca A d1
-        // over the five levels from the end inwards (b0..b4), times 1/betad
-        for (int e = 0; e < 2; ++e) {
-            double* c = ce + (size_t)(2 * k + e) * PE_COUNT;
-            const double sg = e == 0 ? 1.0 : -1.0;               // the top rows are the mirrored ones with the sign changed
-            const int jn = e == 0 ? 1 : nz - 2, je = e == 0 ? 0 : nz - 1;
-            double near[5], end[5] = {0, 0, 0, 0, 0};
-            for (int i = 0; i < 5; ++i) near[i] = sg * cc.Cb[i];
-            const bool closed = e == 0 ? (bc == 1 || bc == 3) : (bc == 1 || bc == 2);
-            if (closed)
-                for (int i = 0; i < 5; ++i)
-                    end[i] = (cc.alpha2 * sg * (i < 4 ? cc.Cf[i] : 0.0) - cc.beta1 * near[i]) * cc.cnst;
-            // d1 of the second row: sg (b2 - b0), of the third: sg (b3 - b1)
-            const double off = e == 0 ? tr.upp[1] : tr.low[nz - 2], off_end = e == 0 ? tr.upp[0] : tr.low[nz - 1];
-            near[2] -= ca * sg; near[0] += ca * sg;
-            near[3] -= ca * sg * off; near[1] += ca * sg * off;
-            end[2] -= ca * sg * off_end; end[0] += ca * sg * off_end;
-            for (int i = 0; i < 5; ++i) {
-                c[i] = near[i] * r.ibd[jn];
-                c[5 + i] = end[i] * r.ibd[je];
-            }
-            c[PE_TOP] = (e == 1 && bc == 3) ? r.ibd[je] : 0.0;
-        }
+        for (int e = 0; e < 2; ++e) closure_row(ce + (size_t)(2 * k + e) * PE_COUNT, e, nz, bc, tr, r.ibd, cc);
         double* c = tab.data() + (size_t)PZ_COUNT * nzp + (size_t)k * PC_COUNT * tp;
         auto Mc = [&](int t) { return r.HH[(size_t)t * ch + ch - 1]; };
         auto Gc = [&](int t) { return r.GG[(size_t)t * ch]; };
@@ -510,6 +548,11 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
         if ((c->use_pencil || c->use_fused) &&
             (rc = dalloc(c, &c->src_plane, (size_t)FUSED_STEPS * c->S * c->M * cs))) return bail(rc);
     }
+    if (mhd_form) {
+        const size_t nt = 4 * (size_t)z_code_size(c->nz);
+        if ((rc = dalloc(c, (void**)&c->ztab64, nt * 8))) return bail(rc);
+        if (c->f32 && (rc = dalloc(c, &c->ztab, nt * 4))) return bail(rc);
+    }
     // twiddle tables: n FP64 values, then the same n values in FP32
     if ((rc = dalloc(c, (void**)&c->tw_x, (size_t)p->nx * 12))) return bail(rc);
     if ((rc = dalloc(c, (void**)&c->tw_y, (size_t)std::max(p->ny, 2) * 12))) return bail(rc);
@@ -522,7 +565,7 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     launch_set_time(c->d_time, 0, c->stream);
     c->t0.assign(c->S, 0);
     c->active_n = c->S;
-    c->use_graphs = getenv("SPARC_NO_GRAPHS") == nullptr && !mhd_form;
+    c->use_graphs = getenv("SPARC_NO_GRAPHS") == nullptr && (!mhd_form || mhd_graphs(c));
     if (c->use_fused) fused_prepare(c->nz, c->nzpml);
     if (mhd_form && (rc = mhd_create(c))) return bail(rc);
     // twiddles cos/sin(2 pi q / n), q < n/2, exact pi; the FP32 copy (rounded
@@ -742,6 +785,13 @@ int sparc_gpu_set_background(sparc_ctx* c, const double* zin, const double* cin,
         }
     }
     int rc;
+    if (c->mhd) {
+        const std::vector<double> tab = z_table(nz, stretch, tri, c->cc64);
+        const std::vector<float> tf(tab.begin(), tab.end());
+        if ((rc = upload(c, c->ztab64, tab.data(), tab.size() * 8)) ||
+            (c->f32 && (rc = upload(c, c->ztab, tf.data(), tf.size() * 4))) || (rc = mhd_set_tables(c)))
+            return rc;      // mhd_set_tables waits for the uploads
+    }
     if (c->use_pencil) {
         const std::vector<double> tab = pencil_table(nz, P.npmlbot, P.npmltop, c->pencil, P.option, c->zt_host.data(), tri, c->cc64);
         if (c->f32) {
@@ -1123,6 +1173,7 @@ static void make_args(sparc_ctx* c, StageArgs<T>& A, UpdateArgs<T>& U) {
 // gate), from the device time, so the same sequence is valid at any time.
 template <typename T>
 static int enqueue_steps(sparc_ctx* c, int nsteps) {
+    if (c->mhd) return mhd_enqueue(c, nsteps);
     StageArgs<T> A;
     UpdateArgs<T> U;
     make_args<T>(c, A, U);
@@ -1239,13 +1290,17 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
 template <typename T>
 static int do_steps(sparc_ctx* c, int nsteps) {
     if (nsteps == 0) return SPARC_OK;
-    if (c->mhd) return mhd_steps(c, nsteps);
+    if (c->mhd) {
+        const int rc = mhd_ready(c);
+        if (rc) return rc;
+    }
     // A long call replays one graph of kGraphChunk steps (every kernel reads
     // the clock on the device, so a captured chunk is valid at any time) and
     // a graph of the remainder: capture and instantiation stay bounded.  Each
     // chunk's last step also writes scr; the call's last step is still the
-    // last to write it.
-    constexpr int kGraphChunk = 64;
+    // last to write it.  A magnetic step is some sixty launches, so its chunk is
+    // shorter.
+    const int kGraphChunk = c->mhd ? 4 : 64;
     if (c->use_graphs && nsteps > kGraphChunk) {
         for (int i = 0; i < nsteps / kGraphChunk; ++i) {
             const int rc = do_steps<T>(c, kGraphChunk);
@@ -1526,7 +1581,6 @@ int sparc_gpu_set_stream_priority(sparc_ctx* c, int level) {
     cudaStreamDestroy(c->stream);
     c->stream = ns;
     c->epoch++;                         // step graphs are captured again on first use
-    if (c->mhd) return mhd_set_stream_priority(c, pr);
     return SPARC_OK;
 }
 

@@ -51,6 +51,7 @@ struct sparc_ctx {
     int stage_q = 1, stage_chunk = 0;             // FP64 stage: lanes per pencil and levels per lane
     void* zc = nullptr;                           // their chunk products of the multipliers (4 rows of nz)
     double* zt64 = nullptr; double* pt64 = nullptr;
+    void* ztab = nullptr; double* ztab64 = nullptr;   // magnetic forms: z-solve tables (zsolve.cuh), T and FP64
     double* tw_x = nullptr; double* tw_y = nullptr;
     void* tmp = nullptr;          // FFT intermediate, nz*M complex T
     void* phys = nullptr;         // one physical field, N reals T
@@ -151,11 +152,13 @@ template <typename T> typename CplxOf<T>::type* CP(void* p) { return (typename C
 // option 10 (mhd.cu)
 int mhd_create(sparc_ctx* c);
 void mhd_destroy(sparc_ctx* c);
-int mhd_set_stream_priority(sparc_ctx* c, int cuda_priority);   // the second stream's priority
 int mhd_set_background(sparc_ctx* c, const double* rho, const double* cs, const double* p, const double* bx,
                        const double* by, const double* bz);
 int mhd2d_set_background(sparc_ctx* c, const double* p, const double* rho, const double* cs, const double* psi);
-int mhd_steps(sparc_ctx* c, int nsteps);
+int mhd_set_tables(sparc_ctx* c);       // from set_background
+int mhd_ready(sparc_ctx* c);            // SPARC_ESTATE without a magnetic background
+bool mhd_graphs(const sparc_ctx* c);    // whether its steps can be captured
+int mhd_enqueue(sparc_ctx* c, int nsteps);
 // sensitivity kernels of option 18 (mhd.cu)
 int mhd2d_derive(sparc_ctx* c, int s0, int G, bool adjoint, void* out, long long ofs);
 int mhd2d_kernel_b_reset(sparc_ctx* c);

@@ -35,11 +35,23 @@ struct LineGate {
 
 static inline bool line_ok(int n) { return n >= 16 && n <= 1024 && (n & (n - 1)) == 0; }
 
-// d/dx of rows of nx reals, or with a real multiplier their filter: nrows rows
-// per field; mul[nx] the derivative's factors of i, or the filter's factors
+// Per field of a list of rows: the factors mul[nx] of the spectrum, times i
+// (a derivative) or real (a filter)
+template <typename T> struct LineMul {
+    const T* mul[LINE_FIELDS];
+    int real;           // bit i: field i's factors are real
+};
+template <typename T> LineMul<T> line_mul(const T* mul, bool real = false) {
+    LineMul<T> m;
+    for (const T*& p : m.mul) p = mul;
+    m.real = real ? -1 : 0;
+    return m;
+}
+
+// d/dx or a filter of rows of nx reals, nrows rows per field
 template <typename T>
-void line_rows(const LineList<T, T>& L, int nsrc, int nx, long long nrows, const T* mul, bool real_mul,
-               const double* tw, const LineGate& gate, cudaStream_t s);
+void line_rows(const LineList<T, T>& L, int nsrc, int nx, long long nrows, const LineMul<T>& mul, const double* tw,
+               const LineGate& gate, cudaStream_t s);
 // d/dy of dense (ny, nx) planes
 template <typename T>
 void line_cols_deriv(const LineList<T, T>& L, int nsrc, int nx, int ny, long long nplanes, const T* mul,

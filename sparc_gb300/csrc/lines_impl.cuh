@@ -110,7 +110,6 @@ template <typename T, typename CT, bool INV> __device__ __forceinline__ void dft
 
 template <int N> struct Plan {
     static constexpr int R1 = N >= 512 ? 32 : N >= 128 ? 16 : N >= 32 ? 8 : 4, R2 = N / R1, TL = R2, G = R1 / R2;
-    static constexpr int LPC = 256 / TL;                // lines (or packed pairs of lines) of a 256-thread CTA
 };
 
 // times W_N^(-+ q), q < N
@@ -168,8 +167,9 @@ __device__ __forceinline__ bool gated_off(const LineGate& g) {
 
 // forward, i mul (or mul), inverse of rows of N reals, two rows packed as the
 // real and imaginary part of a line: both multipliers act on the parts separately
-template <typename T, int N, bool REAL>
-__global__ void __launch_bounds__(256) rows_kernel(const LineList<T, T> L, long long nrows, const T* __restrict__ mul,
+// KIND 0: all fields derivatives; 1: all filters; 2: some of each
+template <typename T, int N, int KIND>
+__global__ void __launch_bounds__(256) rows_kernel(const LineList<T, T> L, long long nrows, const LineMul<T> M,
                                                    const double* __restrict__ tw, const LineGate gate) {
     typedef typename CplxOf<T>::type CT;
     typedef Plan<N> P;
@@ -180,7 +180,9 @@ __global__ void __launch_bounds__(256) rows_kernel(const LineList<T, T> L, long 
     auto zs = [&](int k1, int n2) -> CT& { return Z[k1 * (P::R2 + 1) + n2]; };
     const T* in = L.in[blockIdx.y] + blockIdx.z * L.in_ss;
     T* out = L.out[blockIdx.y] + blockIdx.z * L.out_ss;
-    const long long r0 = 2LL * ((long long)blockIdx.x * P::LPC + pp), r1 = r0 + 1;
+    const T* __restrict__ mul = M.mul[blockIdx.y];
+    const bool real = KIND == 2 ? (M.real >> blockIdx.y) & 1 : KIND == 1;
+    const long long r0 = 2LL * ((long long)blockIdx.x * (blockDim.x / P::TL) + pp), r1 = r0 + 1;
     const bool has0 = r0 < nrows, has1 = r1 < nrows;
     CT v[P::R1];
     #pragma unroll
@@ -196,8 +198,8 @@ __global__ void __launch_bounds__(256) rows_kernel(const LineList<T, T> L, long 
         for (int k2 = 0; k2 < P::R2; ++k2) {
             const T m = __ldg(&mul[t + P::R2 * g + P::R1 * k2]);
             const CT X = v[g * P::R2 + k2];
-            v[g * P::R2 + k2].x = REAL ? m * X.x : -m * X.y;
-            v[g * P::R2 + k2].y = REAL ? m * X.y : m * X.x;
+            v[g * P::R2 + k2].x = m * (real ? X.x : -X.y);
+            v[g * P::R2 + k2].y = m * (real ? X.y : X.x);
         }
     line_mirror<true, N, T>(v, t, zs, tw);
     #pragma unroll
@@ -207,14 +209,13 @@ __global__ void __launch_bounds__(256) rows_kernel(const LineList<T, T> L, long 
     }
 }
 
-// d/dy of dense (N, nx) planes: LPC pairs of adjacent columns per CTA, a pair
+// d/dy of dense (N, nx) planes: NC pairs of adjacent columns per CTA, a pair
 // read and written as one complex value
-template <typename T, int N>
+template <typename T, int N, int NC>
 __global__ void __launch_bounds__(256) cols_deriv_kernel(const LineList<T, T> L, int nx, const T* __restrict__ mul,
                                                          const double* __restrict__ tw) {
     typedef typename CplxOf<T>::type CT;
     typedef Plan<N> P;
-    constexpr int NC = P::LPC;
     extern __shared__ __align__(16) unsigned char smraw[];
     CT* Z = (CT*)smraw;
     const int npair = nx / 2, ntile = (npair + NC - 1) / NC;
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(256) r2c_kernel(const LineList<T, typename Cpl
     auto zs = [&](int k1, int n2) -> CT& { return Z[k1 * (P::R2 + 1) + n2]; };
     const T* in = L.in[blockIdx.y] + blockIdx.z * L.in_ss;
     CT* out = L.out[blockIdx.y] + blockIdx.z * L.out_ss;
-    const long long r0 = 2LL * ((long long)blockIdx.x * P::LPC + pp), r1 = r0 + 1;
+    const long long r0 = 2LL * ((long long)blockIdx.x * (blockDim.x / P::TL) + pp), r1 = r0 + 1;
     const bool has0 = r0 < nrows, has1 = r1 < nrows;
     CT v[P::R1];
     #pragma unroll
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(256) c2r_kernel(const LineList<typename CplxOf
     auto zs = [&](int k1, int n2) -> CT& { return Z[k1 * (P::R2 + 1) + n2]; };
     const CT* in = L.in[blockIdx.y] + blockIdx.z * L.in_ss;
     T* out = L.out[blockIdx.y] + blockIdx.z * L.out_ss;
-    const long long r0 = 2LL * ((long long)blockIdx.x * P::LPC + pp), r1 = r0 + 1;
+    const long long r0 = 2LL * ((long long)blockIdx.x * (blockDim.x / P::TL) + pp), r1 = r0 + 1;
     const bool has0 = r0 < nrows, has1 = r1 < nrows;
     const long long pe = (long long)ny * H;
     const long long o0 = has0 ? grp_off(r0 / ny, ppg, gstride, pe) + (r0 % ny) * H : 0;
@@ -329,15 +330,14 @@ __global__ void __launch_bounds__(256) c2r_kernel(const LineList<typename CplxOf
         }
 }
 
-// complex columns along y, LPC columns per CTA
-template <typename T, int N, bool INV>
+// complex columns along y, NC per CTA
+template <typename T, int N, bool INV, int NC>
 __global__ void __launch_bounds__(256) cols_kernel(const typename CplxOf<T>::type* __restrict__ in,
                                                    typename CplxOf<T>::type* __restrict__ out, int H, int ppg,
                                                    long long gstride, const T* __restrict__ mul,
                                                    const double* __restrict__ tw) {
     typedef typename CplxOf<T>::type CT;
     typedef Plan<N> P;
-    constexpr int NC = P::LPC;
     extern __shared__ __align__(16) unsigned char smraw[];
     CT* Z = (CT*)smraw;
     const int ntile = (H + NC - 1) / NC;
@@ -365,13 +365,12 @@ __global__ void __launch_bounds__(256) cols_kernel(const typename CplxOf<T>::typ
     }
 }
 
-template <typename T, int N>
+template <typename T, int N, int NC>
 __global__ void __launch_bounds__(256) cols_filter_kernel(
     const LineList<typename CplxOf<T>::type, typename CplxOf<T>::type> L, int H, const T* __restrict__ mul,
     const double* __restrict__ tw, const LineGate gate) {
     typedef typename CplxOf<T>::type CT;
     typedef Plan<N> P;
-    constexpr int NC = P::LPC;
     extern __shared__ __align__(16) unsigned char smraw[];
     if (gated_off(gate)) return;
     CT* Z = (CT*)smraw;
@@ -418,21 +417,57 @@ template <typename F> void by_size(int n, F f) {
 template <typename K> void smem_of(K k, size_t bytes) {
     if (bytes > 48 * 1024) cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
-template <int N, typename CT> constexpr size_t row_smem() { return (size_t)Plan<N>::LPC * Plan<N>::R1 * (Plan<N>::R2 + 1) * sizeof(CT); }
-template <int N, typename CT> constexpr size_t col_smem() { return (size_t)Plan<N>::LPC * N * sizeof(CT); }
-inline unsigned row_ctas(long long nrows, int lpc) { return (unsigned)((nrows + 2LL * lpc - 1) / (2LL * lpc)); }
+
+// SMs of the device
+int sm_count() {
+    static const int n = [] {
+        int dev = 0, v = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) v = 0;
+        cudaGetLastError();
+        return v > 0 ? v : 152;
+    }();
+    return n;
+}
+// A launch over row pairs: CTAs, threads and exchange bytes.  Two warps (their
+// barriers cost least: 256x256x300 FP32 d/dx 33 -> 30 us, FP64 the same as
+// larger CTAs); one while the launch would leave an SM with less than four CTAs
+// -- a few lines of FP64 keep an SM's pipe busy for tens of microseconds, so
+// they have to be spread (300 rows of 256: 60 -> 29 us)
+template <int N, typename CT> struct RowLaunch {
+    int b;
+    unsigned ctas;
+    size_t smem;
+    RowLaunch(long long nrows, int batch) {
+        const long long pairs = (nrows + 1) / 2;
+        b = pairs * batch / (64 / Plan<N>::TL) < 4LL * sm_count() ? 32 : 64;
+        const int per = b / Plan<N>::TL;
+        ctas = (unsigned)((pairs + per - 1) / per);
+        smem = (size_t)per * Plan<N>::R1 * (Plan<N>::R2 + 1) * sizeof(CT);
+    }
+};
+// Columns (or pairs) per CTA: rows of 128 bytes, two warps at least.  Wider
+// CTAs waste columns of the nx/2+1 of a half spectrum (FP64, 65 columns: 32 a
+// CTA 154 us, 8 a CTA 126 us); on the nx/2 pairs of a plane there is no such
+// waste and 256 threads are the faster ones (FP64 128: 104 against 100 us)
+template <int N, typename CT> constexpr int narrow() {
+    const int least = sizeof(CT) == 16 || Plan<N>::TL == 32 ? 8 : 16;
+    return least > 64 / Plan<N>::TL ? least : 64 / Plan<N>::TL;
+}
+template <int N> constexpr int wide() { return 256 / Plan<N>::TL; }
 
 }  // namespace
 
 template <typename T>
-void line_rows(const LineList<T, T>& L, int nsrc, int nx, long long nrows, const T* mul, bool real_mul,
-               const double* tw, const LineGate& gate, cudaStream_t s) {
+void line_rows(const LineList<T, T>& L, int nsrc, int nx, long long nrows, const LineMul<T>& mul, const double* tw,
+               const LineGate& gate, cudaStream_t s) {
     typedef typename CplxOf<T>::type CT;
     by_size(nx, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        auto k = real_mul ? rows_kernel<T, N, true> : rows_kernel<T, N, false>;
-        smem_of(k, row_smem<N, CT>());
-        k<<<dim3(row_ctas(nrows, Plan<N>::LPC), L.n, nsrc), 256, row_smem<N, CT>(), s>>>(L, nrows, mul, tw, gate);
+        const int all = (1 << L.n) - 1, kind = (mul.real & all) == 0 ? 0 : (mul.real & all) == all ? 1 : 2;
+        auto k = kind == 0 ? rows_kernel<T, N, 0> : kind == 1 ? rows_kernel<T, N, 1> : rows_kernel<T, N, 2>;
+        const RowLaunch<N, CT> g(nrows, L.n * nsrc);
+        smem_of(k, g.smem);
+        k<<<dim3(g.ctas, L.n, nsrc), g.b, g.smem, s>>>(L, nrows, mul, tw, gate);
     });
 }
 template <typename T>
@@ -441,9 +476,13 @@ void line_cols_deriv(const LineList<T, T>& L, int nsrc, int nx, int ny, long lon
     typedef typename CplxOf<T>::type CT;
     by_size(ny, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        smem_of(cols_deriv_kernel<T, N>, col_smem<N, CT>());
-        const long long tiles = (nx / 2 + Plan<N>::LPC - 1) / Plan<N>::LPC;
-        cols_deriv_kernel<T, N><<<dim3((unsigned)(nplanes * tiles), L.n, nsrc), 256, col_smem<N, CT>(), s>>>(L, nx, mul, tw);
+        auto launch = [&](auto k, int NC) {
+            const long long tiles = (nx / 2 + NC - 1) / NC;
+            smem_of(k, (size_t)NC * N * sizeof(CT));
+            k<<<dim3((unsigned)(nplanes * tiles), L.n, nsrc), NC * Plan<N>::TL, (size_t)NC * N * sizeof(CT), s>>>(L, nx, mul, tw);
+        };
+        if (nplanes * (nx / 2) / wide<N>() * L.n * nsrc >= 4LL * sm_count()) launch(cols_deriv_kernel<T, N, wide<N>()>, wide<N>());
+        else launch(cols_deriv_kernel<T, N, narrow<N, CT>()>, narrow<N, CT>());
     });
 }
 template <typename T>
@@ -452,8 +491,9 @@ void line_r2c(const LineList<T, typename CplxOf<T>::type>& L, int nsrc, int nx, 
     typedef typename CplxOf<T>::type CT;
     by_size(nx, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        smem_of(r2c_kernel<T, N>, row_smem<N, CT>());
-        r2c_kernel<T, N><<<dim3(row_ctas(nrows, Plan<N>::LPC), L.n, nsrc), 256, row_smem<N, CT>(), s>>>(L, nrows, scale, tw, gate);
+        const RowLaunch<N, CT> g(nrows, L.n * nsrc);
+        smem_of(r2c_kernel<T, N>, g.smem);
+        r2c_kernel<T, N><<<dim3(g.ctas, L.n, nsrc), g.b, g.smem, s>>>(L, nrows, scale, tw, gate);
     });
 }
 template <typename T>
@@ -462,9 +502,9 @@ void line_c2r(const LineList<typename CplxOf<T>::type, T>& L, int nsrc, int nx, 
     typedef typename CplxOf<T>::type CT;
     by_size(nx, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        smem_of(c2r_kernel<T, N>, row_smem<N, CT>());
-        c2r_kernel<T, N><<<dim3(row_ctas(nrows, Plan<N>::LPC), L.n, nsrc), 256, row_smem<N, CT>(), s>>>(L, nrows, ny, ppg,
-                                                                                                       gstride, tw, gate);
+        const RowLaunch<N, CT> g(nrows, L.n * nsrc);
+        smem_of(c2r_kernel<T, N>, g.smem);
+        c2r_kernel<T, N><<<dim3(g.ctas, L.n, nsrc), g.b, g.smem, s>>>(L, nrows, ny, ppg, gstride, tw, gate);
     });
 }
 template <typename T>
@@ -473,10 +513,12 @@ void line_cols(const typename CplxOf<T>::type* in, typename CplxOf<T>::type* out
     typedef typename CplxOf<T>::type CT;
     by_size(ny, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        auto k = sign > 0 ? cols_kernel<T, N, true> : cols_kernel<T, N, false>;
-        smem_of(k, col_smem<N, CT>());
-        const long long tiles = (H + Plan<N>::LPC - 1) / Plan<N>::LPC;
-        k<<<(unsigned)(nplanes * tiles), 256, col_smem<N, CT>(), s>>>(in, out, H, ppg, gstride, mul, tw);
+        constexpr int NC = narrow<N, CT>();
+        auto k = sign > 0 ? cols_kernel<T, N, true, NC> : cols_kernel<T, N, false, NC>;
+        const size_t smem = (size_t)NC * N * sizeof(CT);
+        smem_of(k, smem);
+        const long long tiles = (H + NC - 1) / NC;
+        k<<<(unsigned)(nplanes * tiles), NC * Plan<N>::TL, smem, s>>>(in, out, H, ppg, gstride, mul, tw);
     });
 }
 template <typename T>
@@ -485,14 +527,16 @@ void line_cols_filter(const LineList<typename CplxOf<T>::type, typename CplxOf<T
     typedef typename CplxOf<T>::type CT;
     by_size(ny, [&](auto n) {
         constexpr int N = decltype(n)::value;
-        smem_of(cols_filter_kernel<T, N>, col_smem<N, CT>());
-        const long long tiles = (H + Plan<N>::LPC - 1) / Plan<N>::LPC;
-        cols_filter_kernel<T, N><<<dim3((unsigned)(nplanes * tiles), L.n, nsrc), 256, col_smem<N, CT>(), s>>>(L, H, mul, tw, gate);
+        constexpr int NC = narrow<N, CT>();
+        const size_t smem = (size_t)NC * N * sizeof(CT);
+        smem_of(cols_filter_kernel<T, N, NC>, smem);
+        const long long tiles = (H + NC - 1) / NC;
+        cols_filter_kernel<T, N, NC><<<dim3((unsigned)(nplanes * tiles), L.n, nsrc), NC * Plan<N>::TL, smem, s>>>(L, H, mul, tw, gate);
     });
 }
 
 #define INST_LINES(T, CT)                                                                                             \
-    template void line_rows<T>(const LineList<T, T>&, int, int, long long, const T*, bool, const double*,             \
+    template void line_rows<T>(const LineList<T, T>&, int, int, long long, const LineMul<T>&, const double*,          \
                                const LineGate&, cudaStream_t);                                                        \
     template void line_cols_deriv<T>(const LineList<T, T>&, int, int, int, long long, const T*, const double*,        \
                                      cudaStream_t);                                                                   \
