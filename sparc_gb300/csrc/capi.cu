@@ -77,7 +77,7 @@ Tri tri_for(int nz, int ibc) {
 struct FusedRows {
     std::vector<double> ibd, mm, HH, gg, GG;
 };
-FusedRows fused_rows(int nz, int nzp, const Tri& t, int ch = FUSED_CH) {
+FusedRows fused_rows(int nz, int nzp, const Tri& t, int ch) {
     FusedRows r;
     r.ibd.assign(nzp, 0.0); r.mm.assign(nzp, 0.0); r.gg.assign(nzp, 0.0); r.HH.assign(nzp, 0.0);
     r.GG.assign(nzp, 0.0);
@@ -101,7 +101,7 @@ FusedRows fused_rows(int nz, int nzp, const Tri& t, int ch = FUSED_CH) {
 // sig(j)/sig(j-1); back substitution y(j) = sig(j) u(j) + g(j) sig(j)/sig(j+1)
 // y(j+1); the chunk products H, G are those of the new multipliers.  Same
 // recurrences, the scale applied inside them (sig = 1 on padding levels).
-FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig, int ch = FUSED_CH) {
+FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig, int ch) {
     FusedRows o = r;
     const int nzp = (int)r.ibd.size();
     for (int j = 0; j < nzp; ++j) {
@@ -123,7 +123,7 @@ FusedRows fused_rows_scaled(const FusedRows& r, const std::vector<double>& sig, 
 // substitution (zero carry from above) to the carry uin from below,
 // K(j) = H(j) + g(j) K(j+1) within the chunk, K(last) = H(last).  The rows
 // keep H's place; the look-back products use H itself.
-std::vector<double> fused_k_row(const FusedRows& r, int ch = FUSED_CH) {
+std::vector<double> fused_k_row(const FusedRows& r, int ch) {
     const int nzp = (int)r.HH.size();
     std::vector<double> K(nzp, 0.0);
     for (int j0 = 0; j0 < nzp; j0 += ch) {
@@ -134,31 +134,31 @@ std::vector<double> fused_k_row(const FusedRows& r, int ch = FUSED_CH) {
     return K;
 }
 
-// Look-back products of the fused step's carries: fwd[4t + i-2] is the
-// product of the chunk multipliers Mc(t-1)..Mc(t-i+1) (i = 2..5), the factor
-// of chunk t-i's value in the carry into chunk t; bwd[4t + i-2] likewise with
-// the backward chunk multipliers Gc(t+1)..Gc(t+i-1) for chunk t+i.  Returns
-// the largest product over FUSED_KB chunks, the factor of the first chunk the
+// Look-back products of carries over the kb nearest chunks of ch levels:
+// fwd[kp t + i-2] is the product of the chunk multipliers Mc(t-1)..Mc(t-i+1)
+// (i = 2..kb), the factor of chunk t-i's value in the carry into chunk t; bwd
+// likewise with the backward chunk multipliers Gc(t+1)..Gc(t+i-1) for chunk t+i.
+// Returns the largest product over kb chunks, the factor of the first chunk the
 // carries leave out, over the chunks that hold real levels (the carries into
 // padding chunks reach no real row: their H and G rows are zero).
-double fused_lookback(const FusedRows& r, int tp, int nz, std::vector<double>& fwd, std::vector<double>& bwd,
-                      int ch = FUSED_CH) {
+double lookback_products(const FusedRows& r, int tp, int nz, int ch, int kb, int kp, std::vector<double>& fwd,
+                         std::vector<double>& bwd) {
     std::vector<double> Mc(tp), Gc(tp);
     for (int t = 0; t < tp; ++t) {
         Mc[t] = r.HH[t * ch + ch - 1];
         Gc[t] = r.GG[t * ch];
     }
-    fwd.assign((size_t)4 * tp, 0.0);
-    bwd.assign((size_t)4 * tp, 0.0);
+    fwd.assign((size_t)kp * tp, 0.0);
+    bwd.assign((size_t)kp * tp, 0.0);
     double worst = 0.0;
     for (int t = 0; t < tp; ++t) {
         double pf = 1.0, pb = 1.0;
-        for (int i = 2; i <= FUSED_KB + 1; ++i) {
+        for (int i = 2; i <= kb + 1; ++i) {
             pf = (t - i + 1 >= 0) ? pf * Mc[t - i + 1] : 0.0;
             pb = (t + i - 1 < tp) ? pb * Gc[t + i - 1] : 0.0;
-            if (i <= FUSED_KB) {
-                fwd[(size_t)4 * t + i - 2] = pf;
-                bwd[(size_t)4 * t + i - 2] = pb;
+            if (i <= kb) {
+                fwd[(size_t)kp * t + i - 2] = pf;
+                bwd[(size_t)kp * t + i - 2] = pb;
             } else if (t * ch < nz) {
                 worst = std::max(worst, std::max(std::fabs(pf), std::fabs(pb)));
             }
@@ -168,12 +168,14 @@ double fused_lookback(const FusedRows& r, int tp, int nz, std::vector<double>& f
 }
 
 // Whether the look-back carries of the fused step are exact to the stated
-// bound for the two boundary codes of a form (xi_z and p')
-bool fused_lookback_ok(int nz, int bcx, int bcp) {
-    const int nzp = fused_nzp(nz), tp = nzp / FUSED_CH;
-    for (int b : {bcx, bcp}) {
+// bound for the two boundary codes of a form (xi_z and p'; d3: option 4, else 17)
+bool fused_lookback_ok(int nz, bool d3) {
+    const int nzp = fused_nzp(nz, d3), ch = fused_shape(nz, d3).ch;
+    for (int b : {d3 ? 1 : 3, d3 ? 0 : 2}) {
         std::vector<double> f, g;
-        if (fused_lookback(fused_rows(nz, nzp, tri_for(nz, b)), tp, nz, f, g) > FUSED_LOOKBACK_BOUND) return false;
+        if (lookback_products(fused_rows(nz, nzp, tri_for(nz, b), ch), fused_chunks(nz), nz, ch, fused_look_back(nz, d3),
+                              fused_look_stride(nz, d3), f, g) > FUSED_LOOKBACK_BOUND)
+            return false;
     }
     return true;
 }
@@ -250,8 +252,7 @@ std::vector<double> z_table(int nz, const std::vector<double>& stretch, const Tr
             t[PS_A * nzp + j] = (j > 0 && j < nz - 1) ? ca * sig[j] : 0.0;
         }
         std::vector<double> f, b;
-        fused_lookback(r, nw, nz, f, b, ZCS);
-        static_assert(ZKB == FUSED_KB, "fused_lookback's chunks");
+        lookback_products(r, nw, nz, ZCS, ZKB, ZKB - 1, f, b);
         std::copy(f.begin(), f.end(), t + PS_COUNT * nzp);
         std::copy(b.begin(), b.end(), t + PS_COUNT * nzp + nw * (ZKB - 1));
         for (int e = 0; e < 2; ++e)
@@ -496,30 +497,39 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     }
     if (c->f32) {
         // the fused step covers the quiet displacement forms (options 4, 17)
-        c->use_fused = fused_supported(c->nz) && (p->option == 4 || p->option == 17) &&
+        c->use_fused = fused_supported(c->nz, p->option == 4) && (p->option == 4 || p->option == 17) &&
                        getenv("SPARC_FP32_PER_STAGE") == nullptr &&
-                       fused_lookback_ok(c->nz, p->option == 4 ? 1 : 3, p->option == 4 ? 0 : 2);
-        // modes per CTA of the fused step before any autotuning: 8 (one
-        // 512-thread CTA per SM) when it fits and the grid still gives every SM
-        // two CTAs, else 4; SPARC_FUSED_MODES forces a shape (a switch the tests
-        // use to compare the variants)
+                       fused_lookback_ok(c->nz, p->option == 4);
+        // modes per CTA of the fused step before any autotuning: 8 (512 threads
+        // at W = 2) when it fits and the grid still gives every SM two CTAs, else
+        // 4.  With 3 levels a thread five CTAs of 4 fit an SM where two of 8 do,
+        // so 8 pays only from four CTAs an SM (64x64x75: two sources, 528 CTAs of 8,
+        // 34 us a step with 4 and 36 with 8; four sources 67 and 65), and not with
+        // two warps a pencil (128x128x180, four sources: 0.445 and 0.471 ms).
+        // SPARC_FUSED_MODES forces a shape (a switch the tests use to compare the
+        // variants)
         {
             int dev = 0, nsm = 152;
             if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
             cudaGetLastError();
             const long long ctas8 = (long long)((c->M + 7) / 8) * S;
-            c->fused_pencils = (fused_fits(8, c->nz, c->nzpml) && ctas8 >= 2LL * nsm) ? 8 : 4;
+            const FusedShape f = fused_shape(c->nz, p->option == 4);
+            const bool eight = f.ch == 3 ? f.W == 1 && ctas8 >= 4LL * nsm : ctas8 >= 2LL * nsm;
+            c->fused_pencils = (eight && fused_fits(8, c->nz, c->nzpml, c->P.option == 4)) ? 8 : 4;
+            // 2 where each of those CTAs still gets an SM of its own (256x1x300 11.5 us
+            // a step against 13.6 with 4, 32x32x300 14.3 and 14.8)
+            if ((long long)((c->M + 1) / 2) * S <= nsm) c->fused_pencils = 2;
         }
         if (const char* e = getenv("SPARC_FUSED_MODES")) {
             const int v = atoi(e);
-            if (v == 2 || v == 4 || (v == 8 && fused_fits(8, c->nz, c->nzpml))) c->fused_pencils = v;
+            if (v == 2 || v == 4 || (v == 8 && fused_fits(8, c->nz, c->nzpml, c->P.option == 4))) c->fused_pencils = v;
         }
         // SPARC_TEST_FUSED_NO_TABLE_COPY: the fused step issues no z-table
         // copy, so its bounded wait runs out with nothing in flight (a switch
         // the tests use to exercise the timeout path)
         c->fused_test_nocopy = getenv("SPARC_TEST_FUSED_NO_TABLE_COPY") != nullptr;
         if (c->use_fused &&
-            (rc = dalloc(c, (void**)&c->ftab, (size_t)FZ_COUNT * fused_nzp(c->nz) * 4))) return bail(rc);
+            (rc = dalloc(c, (void**)&c->ftab, (size_t)fused_table_floats(c->nz, p->option == 4) * 4))) return bail(rc);
         if ((rc = dalloc(c, (void**)&c->zt64, (size_t)ZT_COUNT * c->nz * 8))) return bail(rc);
         if ((rc = dalloc(c, (void**)&c->pt64, (size_t)PT_COUNT * c->M * 8))) return bail(rc);
     } else {
@@ -529,9 +539,7 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     // FP64 quiet forms and the FP32 velocity form: the whole-step kernel of
     // pencil.cu, where a pencil fits its shared memory and its carries are
     // exact; SPARC_STAGE_LANES and SPARC_FP32_PER_STAGE ask for the per-stage
-    // kernels (the tests compare the two).  FP32 options 4 and 17 on more than
-    // 320 levels stay on the per-stage kernels: on some grids (8x4x321) the
-    // scaled solves' FP32 error is up to three times theirs.
+    // kernels (the tests compare the two).
     {
         int dev = 0;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
@@ -566,7 +574,7 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
     c->t0.assign(c->S, 0);
     c->active_n = c->S;
     c->use_graphs = getenv("SPARC_NO_GRAPHS") == nullptr && (!mhd_form || mhd_graphs(c));
-    if (c->use_fused) fused_prepare(c->nz, c->nzpml);
+    if (c->use_fused) fused_prepare(c->nz, c->nzpml, p->option);
     if (mhd_form && (rc = mhd_create(c))) return bail(rc);
     // twiddles cos/sin(2 pi q / n), q < n/2, exact pi; the FP32 copy (rounded
     // from FP64) follows the FP64 table in the same allocation
@@ -808,11 +816,12 @@ int sparc_gpu_set_background(sparc_ctx* c, const double* zin, const double* cin,
             // profile rows (with the buoyancy products g rho0/rho0 and
             // g drho0/dz / rho0 folded), and the LU
             // elimination multipliers of the xi_z and p' boundary codes with
-            // their chunk products (chunks of FUSED_CH levels; padding rows
+            // their chunk products (chunks of fused_shape's levels; padding rows
             // up to NZP carry zero multipliers)
-            const int NZP = fused_nzp(nz);
             const bool d3 = (P.option == 4);
-            std::vector<float> ft((size_t)FZ_COUNT * NZP, 0.f);
+            const int NZP = fused_nzp(nz, d3), ch = fused_shape(nz, d3).ch, tp = fused_chunks(nz);
+            const int kp = fused_look_stride(nz, d3);
+            std::vector<float> ft((size_t)fused_table_floats(nz, d3), 0.f);
             auto put = [&](int row, int j, double v) { ft[(size_t)row * NZP + j] = (float)v; };
             for (int j = 0; j < nz; ++j) {
                 const double ri = ZR(ZT_RHOINV)[j], g = ZR(ZT_G)[j];
@@ -827,22 +836,19 @@ int sparc_gpu_set_background(sparc_ctx* c, const double* zin, const double* cin,
             }
             const int bcs[2] = {d3 ? 1 : 3, d3 ? 0 : 2};
             const int base[2] = {FZ_SX, FZ_SP};
-            const int lbase[2] = {FZ_LX, FZ_LP};
-            const int tp = NZP / FUSED_CH;
             for (int k = 0; k < 2; ++k) {
                 std::vector<double> sig(NZP, 1.0);
                 for (int j = 0; j < nz; ++j) sig[j] = ZR(ZT_STRETCH)[j] * (k == 1 ? ZR(ZT_RHOINV)[j] : 1.0);
-                const FusedRows fr = fused_rows_scaled(fused_rows(nz, NZP, tri[bcs[k]]), sig);
-                const std::vector<double> kk = fused_k_row(fr);
+                const FusedRows fr = fused_rows_scaled(fused_rows(nz, NZP, tri[bcs[k]], ch), sig, ch);
+                const std::vector<double> kk = fused_k_row(fr, ch);
                 const std::vector<double>* rows[5] = {&fr.ibd, &fr.mm, &kk, &fr.gg, &fr.GG};
                 for (int r = 0; r < 5; ++r)
                     for (int j = 0; j < NZP; ++j) put(base[k] + r, j, (*rows[r])[j]);
                 std::vector<double> lf, lb;
-                fused_lookback(fr, tp, nz, lf, lb);
-                for (int i = 0; i < 4 * tp; ++i) {
-                    put(lbase[k], i, lf[i]);
-                    put(lbase[k] + 1, i, lb[i]);
-                }
+                lookback_products(fr, tp, nz, ch, fused_look_back(nz, d3), kp, lf, lb);
+                float* t = ft.data() + (size_t)FZ_ROWS * NZP + (size_t)k * 2 * kp * tp;
+                std::copy(lf.begin(), lf.end(), t);
+                std::copy(lb.begin(), lb.end(), t + (size_t)kp * tp);
             }
             if ((rc = upload(c, c->ftab, ft.data(), ft.size() * 4))) return rc;
         }
@@ -1186,7 +1192,7 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
         Fz.unstr_top = (float)c->zt_host[(size_t)ZT_UNSTRETCH * c->nz + c->nz - 1];
         Fz.fs = c->fs; Fz.ps = c->ps; Fz.M = c->M; Fz.nz = c->nz; Fz.nzpml = c->nzpml;
         Fz.npmlbot = c->P.npmlbot; Fz.npmltop = c->P.npmltop; Fz.option = c->P.option;
-        Fz.damp = A.damp; Fz.W = fused_w(c->nz);
+        Fz.damp = A.damp;
         for (int i = 0; i < 5; ++i) Fz.betas[i] = (float)c->betas[i];
         Fz.dt = (float)c->deltat;
         Fz.cc.C1 = (float)c->cc64.C1; Fz.cc.C2 = (float)c->cc64.C2;
@@ -1403,7 +1409,7 @@ int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step)
     if (steps < 1) return fail(c, SPARC_EINVAL, "steps < 1");
     const bool fused = c->use_fused && c->f32;
     const int cand[3] = {fused ? 4 : 128, fused ? 2 : 64, fused ? 8 : 32};
-    const int ncand = (fused && !fused_fits(8, c->nz, c->nzpml)) ? 2 : 3;
+    const int ncand = (fused && !fused_fits(8, c->nz, c->nzpml, c->P.option == 4)) ? 2 : 3;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));

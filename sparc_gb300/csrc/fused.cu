@@ -8,9 +8,11 @@
 // loading the z tables once and issuing each item's tile copies right after
 // the previous item's stores have read the tile out of shared memory; a launch
 // of several steps has one CTA per item.  Each mode's
-// z-pencil is split into chunks of CH = 5 levels, one chunk per thread:
+// z-pencil is split into chunks of CH = 5 or 3 levels, one chunk per thread:
 // TP = 32*W threads per pencil, W = ceil(nz / 160) warps, and the pencil is
-// padded to NZP = TP*CH levels.
+// padded to NZP = TP*CH levels.  (CH is odd: the stride of a warp's float2
+// accesses; four levels a thread had four-way bank conflicts, 128x128x330 with
+// two sources 0.667 ms a step against 0.422 with five.)
 //   * a (6 fields) lives in shared memory as a tile [field][mode][z] with
 //     zero ghost rows on both ends; global rows [field][z][m0..m0+P-1] are
 //     8P bytes, so the tile is loaded (cp.async, each value into its
@@ -34,8 +36,9 @@
 //     B(t-i) times the product of the multipliers Mc between them (and the
 //     same from above for the back substitution).  Those products depend on
 //     z only (the matrix is the same for every mode), shrink by about 0.008
-//     per chunk (|multiplier| ~ 0.38 per level), and are precomputed on the
-//     host in FP64: the sum is taken over the KB = 5 nearest chunks, read
+//     per chunk of 5 (|multiplier| ~ 0.38 per level), and are precomputed on the
+//     host in FP64: the sum is taken over the KB = 5 nearest chunks (9 of 3
+//     levels; 8 would leave out terms of 2.9e-10, above the bound below), read
 //     from a per-pencil line in shared memory after one barrier.  The terms
 //     left out are below 2^-32 of a chunk value (checked on the host for
 //     every boundary code, else the context runs the per-stage kernels).
@@ -64,16 +67,19 @@
 // HBM traffic per launch: read a, write a (+ the PML planes and source planes),
 // and scr only on steps whose right-hand side is requested (outputs).
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "internal.cuh"
 
 namespace {
 
-constexpr int CH = FUSED_CH;   // z-levels per thread
 constexpr int GZ = 5;          // ghost rows of the tile on each side (reach of the z filter)
 constexpr int GX = 2;          // ghost entries of an exchange line on each side (compact stencil)
-constexpr int KB = FUSED_KB;   // chunks summed by a look-back carry
+// CH z-levels per thread; KB chunks summed by a look-back carry, its products
+// stored KP to a chunk
+__host__ __device__ constexpr int look_back(int ch) { return ch == 3 ? 9 : 5; }
+__host__ __device__ constexpr int look_stride(int ch) { return ch == 3 ? 8 : 4; }
 
 // Entry idx of the z tables (scalars in shared memory) as a pair (t, t), the
 // multiplier of a paired product with a complex value.  Tables stored as
@@ -90,15 +96,23 @@ __device__ __forceinline__ void pencil_sync(int pi, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(pi + 1), "r"(nthreads) : "memory");
 }
 
-// Carry of a chunk from the KB = 5 nearest chunk values of a look-back line:
-// sum over i = 1..5 of prod(i) * v(i), prod(1) = 1, prod(2..5) = pr.x..pr.w,
-// as two independent partial sums (a shorter dependency chain).
-__device__ __forceinline__ float2 lookback(float4 pr, float2 v1, float2 v2, float2 v3, float2 v4, float2 v5) {
-    float2 c1 = pmul(bc2(pr.w), v5);
-    c1 = pfma(bc2(pr.z), v4, c1);
-    float2 c2 = pmul(bc2(pr.y), v3);
-    c2 = pfma(bc2(pr.x), v2, c2);
-    return padd(v1, padd(c1, c2));
+// Carry of a chunk from the KB nearest chunk values of a look-back line, v[0],
+// v[D], v[2 D], ...: v[0] + sum of pr[i] v[(i+1) D], as two independent partial
+// sums (a shorter dependency chain).
+template <int KB, int D>
+__device__ __forceinline__ float2 lookback(const float* pr, const float2* v) {
+    float2 c1 = pmul(bc2(pr[KB - 2]), v[(KB - 1) * D]), c2 = pmul(bc2(pr[(KB - 1) / 2 - 1]), v[(KB - 1) / 2 * D]);
+    #pragma unroll
+    for (int i = KB - 3; i >= (KB - 1) / 2; --i) c1 = pfma(bc2(pr[i]), v[(i + 1) * D], c1);
+    #pragma unroll
+    for (int i = (KB - 1) / 2 - 2; i >= 0; --i) c2 = pfma(bc2(pr[i]), v[(i + 1) * D], c2);
+    return padd(v[0], padd(c1, c2));
+}
+// the products of chunk t
+template <int KP>
+__device__ __forceinline__ void products(const float* tab, int t, float (&pr)[KP]) {
+    #pragma unroll
+    for (int i = 0; i < KP; i += 4) *(float4*)&pr[i] = *(const float4*)(tab + KP * t + i);
 }
 
 // d/dz (without stretch) of the values of one exchange line (xp[j], j in
@@ -106,16 +120,16 @@ __device__ __forceinline__ float2 lookback(float4 pr, float2 v1, float2 v2, floa
 // levels j0..j0+CH-1,
 // boundary code BC (dbyd2.f90:94-173 for the right-hand side; top is the
 // caller-set value of bc 3).  zs, r0: the z tables and the first of the five
-// elimination rows (1/betad, m, K, g, G) of BC; lb, lb+1: its forward and
-// backward look-back product tables ([t][4] floats each); lf, lk:
+// elimination rows (1/betad, m, K, g, G) of BC; lb: its forward and then its
+// backward look-back product tables ([t][KP] floats each); lf, lk:
 // this pencil's forward and backward look-back lines (chunk t at index t,
 // zero entries at -KB..-1 and TP..TP+KB-1).
-template <int BC, int W>
+template <int BC, int W, int CH>
 __device__ __forceinline__ void zsolve(const float2* __restrict__ xp, const float2 (&own)[CH],
-                                       const float* __restrict__ zs, int r0, int lb, int nz, float2 top, int j0,
+                                       const float* __restrict__ zs, int r0, const float* lb, int nz, float2 top, int j0,
                                        bool lo, bool hi, int t, float2* lf, float2* lk, int pi,
                                        const Compact<float> c, float2 (&out)[CH]) {
-    constexpr int NZP = 160 * W;
+    constexpr int NZP = 32 * W * CH, TP = 32 * W, KB = look_back(CH), KP = look_stride(CH);
     const int ibd = r0 * NZP, mm = (r0 + 1) * NZP, HH = (r0 + 2) * NZP, gg = (r0 + 3) * NZP, GG = (r0 + 4) * NZP;
     auto Z = [&](int row, int j) { return zt2(zs, row + j); };
     float2 u[CH];
@@ -126,14 +140,16 @@ __device__ __forceinline__ void zsolve(const float2* __restrict__ xp, const floa
     #pragma unroll
     for (int q = 0; q < CH; ++q) {
         const int j = j0 + q;
-        const float2 bm2 = q >= 2 ? own[q - 2] : xp[j - 2];
-        const float2 bm1 = q >= 1 ? own[q - 1] : xp[j - 1];
-        const float2 bp1 = q + 1 < CH ? own[q + 1] : xp[j + 1];
-        const float2 bp2 = q + 2 < CH ? own[q + 2] : xp[j + 2];
+        const float2 bm2 = q >= 2 ? own[q >= 2 ? q - 2 : 0] : xp[j - 2];
+        const float2 bm1 = q >= 1 ? own[q >= 1 ? q - 1 : 0] : xp[j - 1];
+        const float2 bp1 = q + 1 < CH ? own[q + 1 < CH ? q + 1 : 0] : xp[j + 1];
+        const float2 bp2 = q + 2 < CH ? own[q + 2 < CH ? q + 2 : 0] : xp[j + 2];
         u[q] = pfma(C2p, psub(bp2, bm2), pmul(C1p, psub(bp1, bm1)));
     }
     if (lo) {   // rows 0 and 1 (dbyd2.f90:104-173)
-        const float2 b0 = own[0], b1 = own[1], b2 = own[2], b3 = own[3], b4 = own[4];   // j0 = 0
+        // j0 = 0; levels past the chunk from the line
+        const float2 b0 = own[0], b1 = own[1], b2 = own[2], b3 = CH > 3 ? own[CH > 3 ? 3 : 0] : xp[3];
+        const float2 b4 = CH > 4 ? own[CH > 4 ? 4 : 0] : xp[4];
         const float2 r1 = c.Cb[0] * b0 + c.Cb[1] * b1 + c.Cb[2] * b2 + c.Cb[3] * b3 + c.Cb[4] * b4;
         u[1] = r1;
         if (BC == 0 || BC == 2) {
@@ -170,7 +186,6 @@ __device__ __forceinline__ void zsolve(const float2* __restrict__ xp, const floa
         u[q] = run;
     }
     // carry into the chunk: ud(j0-1) from the chunk values below
-    constexpr int TP = 32 * W;
     lf[t] = run;
     // back substitution x0(j) = u(j) + g(j) x0(j+1) with zero carries, while
     // the other chunks reach the barrier; the carries enter afterwards as
@@ -181,14 +196,15 @@ __device__ __forceinline__ void zsolve(const float2* __restrict__ xp, const floa
         xr = pfma(Z(gg, j0 + q), xr, u[q]);
         out[q] = xr;
     }
-    const float4 prf = *(const float4*)(zs + lb * NZP + 4 * t);      // read before the barrier
+    float pr[KP];
+    products<KP>(lb, t, pr);      // read before the barrier
     pencil_sync(pi, TP);
-    const float2 uin = lookback(prf, lf[t - 1], lf[t - 2], lf[t - 3], lf[t - 4], lf[t - 5]);
+    const float2 uin = lookback<KB, -1>(pr, lf + t - 1);
     // carry from above: x(j0+CH) from the chunk values above
     lk[t] = pfma(Z(HH, j0), uin, xr);
-    const float4 prb = *(const float4*)(zs + (lb + 1) * NZP + 4 * t);
+    products<KP>(lb + TP * KP, t, pr);
     pencil_sync(pi, TP);
-    const float2 xin = lookback(prb, lk[t + 1], lk[t + 2], lk[t + 3], lk[t + 4], lk[t + 5]);
+    const float2 xin = lookback<KB, 1>(pr, lk + t + 1);
     #pragma unroll
     for (int q = 0; q < CH; ++q) out[q] = pfma(Z(GG, j0 + q), xin, pfma(Z(HH, j0 + q), uin, out[q]));
 }
@@ -208,8 +224,9 @@ __device__ __forceinline__ bool mbar_wait(unsigned mbar, int limit) {
 struct FusedLayout {
     int tile, xl, ptile, spt, lines, zs, mbar, total;
 };
-__host__ __device__ inline FusedLayout fused_layout(int P, int W, int nzpml) {
-    const int NZP = 160 * W, LZ = NZP + 2 * GZ, LX = NZP + 2 * GX, LL = 32 * W + 2 * KB;
+__host__ __device__ inline FusedLayout fused_layout(int P, int W, int CH, int nzpml) {
+    const int KB = look_back(CH);
+    const int NZP = 32 * W * CH, LZ = NZP + 2 * GZ, LX = NZP + 2 * GX, LL = 32 * W + 2 * KB;
     FusedLayout L;
     int o = 0;
     L.tile = o;  o += 6 * P * LZ * 8;
@@ -218,7 +235,7 @@ __host__ __device__ inline FusedLayout fused_layout(int P, int W, int nzpml) {
     L.spt = o;   o += 2 * nzpml * P * 8;
     L.lines = o; o += 2 * P * LL * 8;         // forward and backward look-back lines per pencil
     o = (o + 15) & ~15;
-    L.zs = o;    o += FZ_COUNT * NZP * 4;
+    L.zs = o;    o += (FZ_ROWS * NZP + 4 * 32 * W * look_stride(CH)) * 4;
     o = (o + 15) & ~15;
     o = (o + 7) & ~7;
     L.mbar = o;  o += 8;                  // mbarrier of the z-table bulk copy
@@ -228,24 +245,32 @@ __host__ __device__ inline FusedLayout fused_layout(int P, int W, int nzpml) {
 
 }  // namespace
 
+// CTAs of an SM: 16 warps of 128 registers; with 3 levels a thread 20 warps of
+// 96 (24 warps of 80 spill: 64x64x75, two sources, 38.0 us a step against 33.7).
+// W = 3: 12 warps, of which the tiles fit at most.
+__host__ __device__ constexpr int fused_ctas(int P, int W, int CH) {
+    return (CH == 3 ? 20 : 16) / (P * W) > 0 ? (CH == 3 ? 20 : 16) / (P * W) : 1;
+}
+
 // P modes per CTA (2, 4 or 8): every pencil's arithmetic is the same for
-// each, so the results are too; the launch bounds keep 128 registers per
-// thread (P = 8 at W = 2: one 512-thread CTA per SM, the z tables loaded once
-// per eight modes).
-template <bool D3, int W, int P>
-__global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedArgs A) {
+// each, so the results are too (P = 8 at W = 2: one 512-thread CTA per SM, the
+// z tables loaded once per eight modes).
+template <bool D3, int W, int P, int CH>
+__global__ void __launch_bounds__(P * 32 * W, fused_ctas(P, W, CH)) fused_step_kernel(const FusedArgs A) {
     extern __shared__ __align__(16) unsigned char smraw[];
+    constexpr int KB = look_back(CH);
     constexpr int TP = 32 * W, NZP = TP * CH, LZ = NZP + 2 * GZ, LX = NZP + 2 * GX, LL = TP + 2 * KB;
     constexpr int BCX = D3 ? 1 : 3, BCP = D3 ? 0 : 2;
     const int nz = A.nz, M = A.M, nzpml = A.nzpml, nb = A.npmlbot, nt = A.npmltop;
     const long long fs = A.fs;
-    const FusedLayout Ly = fused_layout(P, W, nzpml);
+    const FusedLayout Ly = fused_layout(P, W, CH, nzpml);
     float2* tile = (float2*)(smraw + Ly.tile);            // [6][P][LZ], level j at GZ + j
     float2* xlb = (float2*)(smraw + Ly.xl);               // [P][LX], level j at GX + j
     float2* ptile = (float2*)(smraw + Ly.ptile);          // [2][nzpml][P]
     float2* spt = (float2*)(smraw + Ly.spt);              // [2][nzpml][P] PML right-hand sides
     float2* lines = (float2*)(smraw + Ly.lines);          // [P][2][LL], chunk t at KB + t
-    float* zs = (float*)(smraw + Ly.zs);                  // [FZ_COUNT][NZP]
+    float* zs = (float*)(smraw + Ly.zs);                  // [FZ_ROWS][NZP], look-back products [2][2][TP][KP]
+    const float* lbt = zs + FZ_ROWS * NZP;
     const unsigned mbar = (unsigned)__cvta_generic_to_shared(smraw + Ly.mbar);
     const int nthr = blockDim.x;
     const int pi = threadIdx.x / TP;                      // pencil within the CTA
@@ -263,7 +288,7 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
     // by thread 0 and awaited, with a bounded wait, after the cooperative
     // loads below; 16-byte aligned at both ends, a multiple of 16 bytes ----
     if (threadIdx.x == 0) {
-        const unsigned bytes = FZ_COUNT * NZP * 4;
+        const unsigned bytes = (FZ_ROWS * NZP + 4 * TP * look_stride(CH)) * 4;
         const unsigned dst = (unsigned)__cvta_generic_to_shared(zs);
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(mbar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -426,9 +451,9 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
                 float2 v = TA(2, j0 + q);
                 if (hs) v = pfma(BT, sc[2][q], v);
                 own[q] = v;
-                // level j0+2 is no neighbour's stencil value; only the top rows'
-                // closure (levels nz-5..nz-1) may read it from the line
-                if (q != 2 || j0 + 2 >= nz - 5) xl[j0 + q] = v;
+                // of five levels j0+2 is no neighbour's stencil value; only the top
+                // rows' closure (levels nz-5..nz-1) may read it from the line
+                if (CH != 5 || q != 2 || j0 + 2 >= nz - 5) xl[j0 + q] = v;
             }
             float2 top = make_float2(0.f, 0.f);
             if (!D3 && hi) {   // caller-set top value of bc 3 (physics2d.f90:960)
@@ -443,7 +468,7 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
             pencil_sync(pi, TP);
             float2 d[CH];
             // d: the stretched derivative (the solve's tables carry the stretch)
-            zsolve<BCX, W>(xl, own, zs, FZ_SX, FZ_LX, nz, top, j0, lo, hi, t, lf, lk, pi, A.cc, d);
+            zsolve<BCX, W, CH>(xl, own, zs, FZ_SX, lbt, nz, top, j0, lo, hi, t, lf, lk, pi, A.cc, d);
             if (pml_t) {   // psi_vz (displacement.f90 PML rows)
                 #pragma unroll
                 for (int q = 0; q < CH; ++q) {
@@ -472,13 +497,13 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
                 }
                 const float2 p = pmul(make_float2(-1.f, -1.f), pfma(Z2(FZ_GP, j), xz, pmul(Z2(FZ_C2R, j), div)));
                 qt[q] = pfma(Z2(FZ_E2, j), xz, pmul(Z2(FZ_E1, j), div));   // -g rho'/rho0
-                if (q != 2 || j0 + 2 >= nz - 5) xl[j] = p;
+                if (CH != 5 || q != 2 || j0 + 2 >= nz - 5) xl[j] = p;
                 own[q] = p;
             }
             pencil_sync(pi, TP);
             // ---- dp'/dz, RHS v_z and xi_z ----
             // d: (stretch / rho0) dp'/dz, scaled by the solve's tables
-            zsolve<BCP, W>(xl, own, zs, FZ_SP, FZ_LP, nz, make_float2(0.f, 0.f), j0, lo, hi, t, lf, lk, pi, A.cc, d);
+            zsolve<BCP, W, CH>(xl, own, zs, FZ_SP, lbt + 2 * TP * look_stride(CH), nz, make_float2(0.f, 0.f), j0, lo, hi, t, lf, lk, pi, A.cc, d);
             // ---- horizontal right-hand sides (they do not feed the p' solve) ----
             #pragma unroll
             for (int q = 0; q < CH; ++q) {
@@ -580,9 +605,14 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
             }
             pencil_sync(pi, TP);
             // ---- z filter (+ horizontal filter): field f is filtered into registers,
-            // and written back after the next barrier, while field f+1 is filtered ----
+            // and written back after the next barrier, while field f+1 is filtered.  The
+            // weights (exact in FP32) sum to 1, so in 3-D a level's value is added last:
+            // the partial sums are then small for a smooth field, and the sum rounds
+            // once at the field's size instead of six times (option 4's FP32 error a
+            // quarter smaller).  The 2-D form keeps its order: its FP32 error, 1e-5 to
+            // 5e-5 after a source has acted, comes from v_z in the top rows ----
             const float h1 = 0.5f * 0.41015625f, h2 = 0.5f * -0.234375f, h3 = 0.5f * 0.087890625f;
-            const float h4 = 0.5f * -0.01953125f, h5 = 0.5f * 0.001953125f, c0 = 0.75390625f;
+            const float h4 = 0.5f * -0.01953125f, h5 = 0.5f * 0.001953125f, c0 = 0.75390625f - (D3 ? 1.f : 0.f);
             const bool hfil_on = slot_hfilter(A.clk, tl);
             const float hf = (hfil_on && mvalid) ? A.pt[PT_HF * M + m] : 1.f;
             const bool flo = j0 < 5, fhi = (j0 < nz) && (j0 + CH > nz - 5);
@@ -600,7 +630,8 @@ __global__ void __launch_bounds__(P * 64, 8 / P) fused_step_kernel(const FusedAr
                         acc = pfma(bc2(h2), padd(V[j - 2], V[j + 2]), acc);
                         acc = pfma(bc2(h3), padd(V[j - 3], V[j + 3]), acc);
                         acc = pfma(bc2(h4), padd(V[j - 4], V[j + 4]), acc);
-                        out[q] = pfma(bc2(h5), padd(V[j - 5], V[j + 5]), acc);
+                        acc = pfma(bc2(h5), padd(V[j - 5], V[j + 5]), acc);
+                        out[q] = D3 ? padd(V[j], acc) : acc;
                     }
                     if (flo || fhi) {   // FILTER_VARS_3D / _2D boundary rows
                         #pragma unroll
@@ -731,72 +762,99 @@ template void launch_source_plane<float>(float2*, const float2*, long long, int,
 template void launch_source_plane<double>(double2*, const double2*, long long, int, const SlotClock&, int, int, int,
                                           cudaStream_t);
 
-int fused_w(int nz) { return (nz + 32 * CH - 1) / (32 * CH); }
-int fused_nzp(int nz) { return 32 * CH * fused_w(nz); }
-
-// whether P modes per CTA fit the 227 KB of shared memory a CTA may use
-bool fused_fits(int P, int nz, int nzpml) {
-    return fused_layout(P, fused_w(nz), nzpml).total <= 227 * 1024;
+// Levels per thread and warps per pencil.  A step is bound by the chain of each
+// thread's levels and the barriers between, so the pencil takes the fewest
+// warps that hold it at 5 levels a thread, and 3 levels where those warps hold
+// it at 3 (nz up to 96 and 161 to 192).  Per step with 3 and with 5 levels:
+// 64x64x75, two sources, 34 and 43 us; 256x256x75, four sources, 0.96 and 1.16
+// ms; 128x128x180, four sources, 0.44 and 0.53 ms.  With three warps (321 to 480
+// levels, the per-stage kernels before): 256x256x400 11.7 -> 0.83 ms.
+// The 2-D form stays at 5 levels and two warps at most: another order of its
+// sums moves its FP32 results by the 1e-5 to 5e-5 that rounding leaves of them.
+FusedShape fused_shape(int nz, bool d3) {
+    const int W = nz <= 160 ? 1 : nz <= 320 ? 2 : 3;
+    return {d3 && nz <= 96 * W && W < 3 ? 3 : 5, W};
+}
+int fused_nzp(int nz, bool d3) {
+    const FusedShape f = fused_shape(nz, d3);
+    return 32 * f.W * f.ch;
+}
+int fused_chunks(int nz) { return 32 * fused_shape(nz, true).W; }
+int fused_look_back(int nz, bool d3) { return look_back(fused_shape(nz, d3).ch); }
+int fused_look_stride(int nz, bool d3) { return look_stride(fused_shape(nz, d3).ch); }
+int fused_table_floats(int nz, bool d3) {
+    return FZ_ROWS * fused_nzp(nz, d3) + 4 * fused_chunks(nz) * fused_look_stride(nz, d3);
 }
 
-size_t fused_smem_bytes(int nz, int nzpml, int W) {
-    (void)nz;
-    return (size_t)fused_layout(4, W, nzpml).total;
+// whether P modes per CTA are built (512 threads at most) and fit the 227 KB of shared memory
+bool fused_fits(int P, int nz, int nzpml, bool d3) {
+    const FusedShape f = fused_shape(nz, d3);
+    return P * 32 * f.W <= 512 && fused_layout(P, f.W, f.ch, nzpml).total <= 227 * 1024;
 }
 
 // nz >= 16 keeps the boundary rows of the two ends in different threads
-int fused_supported(int nz) { return nz >= 16 && nz <= 2 * 32 * CH; }
+int fused_supported(int nz, bool d3) { return nz >= 16 && nz <= (d3 ? 480 : 320); }
 
-template <bool D3, int W, int P>
-static void fused_attr(int nzpml) {
-    const size_t sm = (size_t)fused_layout(P, W, nzpml).total;
-    cudaFuncSetAttribute((const void*)fused_step_kernel<D3, W, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sm);
-}
+namespace {
 
-// Dynamic shared-memory limits of every variant a context may launch, set
-// once at context creation (not while a launch sequence is being captured).
-void fused_prepare(int nz, int nzpml) {
-    const int W = fused_w(nz);
-    if (W == 1) {
-        fused_attr<true, 1, 2>(nzpml); fused_attr<true, 1, 4>(nzpml); fused_attr<true, 1, 8>(nzpml);
-        fused_attr<false, 1, 2>(nzpml); fused_attr<false, 1, 4>(nzpml); fused_attr<false, 1, 8>(nzpml);
-    } else {
-        fused_attr<true, 2, 2>(nzpml); fused_attr<true, 2, 4>(nzpml); fused_attr<true, 2, 8>(nzpml);
-        fused_attr<false, 2, 2>(nzpml); fused_attr<false, 2, 4>(nzpml); fused_attr<false, 2, 8>(nzpml);
-    }
-}
-
-template <bool D3, int W, int P>
-static void launch_fused_t(const FusedArgs& A, int nsrc, cudaStream_t s) {
-    const size_t sm = (size_t)fused_layout(P, W, A.nzpml).total;
+template <bool D3, int W, int P, int CH>
+int launch_fused_t(const FusedArgs& A, int nsrc, bool prepare, cudaStream_t s) {
+    const size_t sm = (size_t)fused_layout(P, W, CH, A.nzpml).total;
+    if (prepare)
+        return cudaFuncSetAttribute((const void*)fused_step_kernel<D3, W, P, CH>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
     FusedArgs B = A;
     B.nsrc = nsrc;
     int dev = 0, nsm = 0, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fused_step_kernel<D3, W, P>, P * 32 * W, sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fused_step_kernel<D3, W, P, CH>, P * 32 * W, sm);
     const long long items = (long long)((A.M + P - 1) / P) * nsrc;
     const long long resident = (long long)std::max(nsm, 1) * std::max(occ, 1);
     // one step: one CTA per resident slot, looping over the items (its z tables
     // are loaded once).  Several steps: one CTA per item, so that a launch of
     // another stream gets SMs as the items end.
     const int ncta = (int)(A.nsteps > 1 ? items : std::min(items, resident));
-    fused_step_kernel<D3, W, P><<<ncta, P * 32 * W, sm, s>>>(B);
+    fused_step_kernel<D3, W, P, CH><<<ncta, P * 32 * W, sm, s>>>(B);
+    return 1;
 }
 
-template <bool D3, int W>
-static void launch_fused_p(const FusedArgs& A, int nsrc, cudaStream_t s) {
-    if (A.pencils == 2) launch_fused_t<D3, W, 2>(A, nsrc, s);
-    else if (A.pencils == 8) launch_fused_t<D3, W, 8>(A, nsrc, s);
-    else launch_fused_t<D3, W, 4>(A, nsrc, s);
+template <bool D3, int W, int CH>
+int launch_fused_p(const FusedArgs& A, int nsrc, bool prepare, cudaStream_t s) {
+    if (A.pencils == 2) return launch_fused_t<D3, W, 2, CH>(A, nsrc, prepare, s);
+    if (A.pencils == 4) return launch_fused_t<D3, W, 4, CH>(A, nsrc, prepare, s);
+    if constexpr (W < 3) return launch_fused_t<D3, W, 8, CH>(A, nsrc, prepare, s);
+    return 0;
+}
+
+template <bool D3>
+int launch_fused_w(const FusedArgs& A, int nsrc, bool prepare, cudaStream_t s) {
+    const FusedShape f = fused_shape(A.nz, D3);
+    if constexpr (D3) {
+        if (f.ch == 3) return f.W == 1 ? launch_fused_p<D3, 1, 3>(A, nsrc, prepare, s) : launch_fused_p<D3, 2, 3>(A, nsrc, prepare, s);
+        if (f.W == 3) return launch_fused_p<D3, 3, 5>(A, nsrc, prepare, s);
+    }
+    return f.W == 1 ? launch_fused_p<D3, 1, 5>(A, nsrc, prepare, s) : launch_fused_p<D3, 2, 5>(A, nsrc, prepare, s);
+}
+
+}  // namespace
+
+// Dynamic shared-memory limits of every variant a context may launch, set
+// once at context creation (not while a launch sequence is being captured).
+void fused_prepare(int nz, int nzpml, int option) {
+    FusedArgs A;
+    memset(&A, 0, sizeof(A));
+    A.nz = nz;
+    A.nzpml = nzpml;
+    for (int P : {2, 4, 8}) {
+        A.pencils = P;
+        if (!fused_fits(P, nz, nzpml, option == 4)) continue;
+        if (option == 4) launch_fused_w<true>(A, 1, true, nullptr);
+        else launch_fused_w<false>(A, 1, true, nullptr);
+    }
 }
 
 void launch_fused(const FusedArgs& A, int nsrc, cudaStream_t s) {
-    const bool d3 = (A.option == 4);
-    if (A.W == 1) {
-        if (d3) launch_fused_p<true, 1>(A, nsrc, s); else launch_fused_p<false, 1>(A, nsrc, s);
-    } else {
-        if (d3) launch_fused_p<true, 2>(A, nsrc, s); else launch_fused_p<false, 2>(A, nsrc, s);
-    }
+    if (A.option == 4) launch_fused_w<true>(A, nsrc, false, s);
+    else launch_fused_w<false>(A, nsrc, false, s);
 }

@@ -313,24 +313,24 @@ template <typename T> struct UpdateArgs {
 };
 
 // fused FP32 step (fused.cu)
-// z table of the fused FP32 step, [FZ_COUNT][NZP] (NZP = fused_nzp(nz), padded
+// z table of the fused FP32 step, [FZ_ROWS][NZP] (NZP = fused_nzp, padded
 // rows zero): profile rows, then the five elimination rows (1/betad,
 // elimination multiplier m, the carry response K = H + g K(next) of the
 // chunk's back substitution, H the chunk products of m, back-substitution
 // multiplier g, chunk products G of g) of the xi_z boundary code and of the p'
-// boundary code, then the look-back products of each code: a forward row and
-// a backward row, [chunk t][4] floats each (the products of the multipliers
-// of the 1..4 chunks between chunk t and the chunk 2..5 below / above it).
+// boundary code; then the look-back products of each code: a forward and a
+// backward table, [chunk t][KP] floats each (the products of the multipliers of
+// the 1..KB-1 chunks between chunk t and the chunk 2..KB below / above it;
+// KB = fused_look_back, KP = fused_look_stride).
 // The elimination rows solve for s(j) x(j) instead of x(j), s = stretch for
 // xi_z and stretch / rho0 for p' (the factors the step applies to the two
 // derivatives): 1/betad and the multipliers carry the ratios of s, so the
 // solves return the scaled derivatives directly.
 enum {
     FZ_AZR = 0, FZ_C2R, FZ_GP, FZ_RI, FZ_E1, FZ_E2, FZ_AZ, FZ_BZ, FZ_SX = 8, FZ_SP = 13,
-    FZ_LX = 18, FZ_LP = 20, FZ_COUNT = 22
+    FZ_ROWS = 18
 };
-constexpr int FUSED_KB = 5;    // chunks summed by a look-back carry of the fused step
-// largest product of chunk multipliers over FUSED_KB chunks (the first term a
+// largest product of chunk multipliers over a carry's chunks (the first term a
 // look-back carry leaves out) for which the fused step is used
 constexpr double FUSED_LOOKBACK_BOUND = 2.3283064365386963e-10;   // 2^-32
 struct FusedArgs {
@@ -338,7 +338,7 @@ struct FusedArgs {
     const float* ftab; const float* pt;
     float unstr_top;
     long long fs, ps;
-    int M, nz, nzpml, npmlbot, npmltop, option, damp, W;
+    int M, nz, nzpml, npmlbot, npmltop, option, damp;
     float betas[5];
     float dt;
     Compact<float> cc;
@@ -360,14 +360,17 @@ struct FusedArgs {
     int pf_stride;      // > 0: each CTA prefetches into L2 the rows of the CTA pf_stride later in launch
                         // order (set by the launcher to the CTAs resident at once); 0: no prefetch
 };
-constexpr int FUSED_CH = 5;
-constexpr int FUSED_STEPS = 16;   // time steps of one launch of the fused step, at most
-void fused_prepare(int nz, int nzpml);
-size_t fused_smem_bytes(int nz, int nzpml, int W);
-bool fused_fits(int P, int nz, int nzpml);
-int fused_supported(int nz);
-int fused_w(int nz);
-int fused_nzp(int nz);
+constexpr int FUSED_STEPS = 16;   // time steps of one launch of the whole-step kernels, at most
+struct FusedShape { int ch, W; }; // levels per thread, warps per pencil
+FusedShape fused_shape(int nz, bool d3);   // d3: option 4, else 17
+int fused_nzp(int nz, bool d3);            // padded levels
+int fused_chunks(int nz);
+int fused_look_back(int nz, bool d3);      // chunks summed by a carry, and floats per chunk of its product tables
+int fused_look_stride(int nz, bool d3);
+int fused_table_floats(int nz, bool d3);
+void fused_prepare(int nz, int nzpml, int option);
+bool fused_fits(int P, int nz, int nzpml, bool d3);
+int fused_supported(int nz, bool d3);
 void launch_fused(const FusedArgs& A, int nsrc, cudaStream_t s);
 
 // whole-step kernel on pencils (pencil.cu).  Table [PZ_COUNT][NZP], level

@@ -123,7 +123,8 @@ class Solver:
         choice = ctypes.c_int(0)
         ms = ctypes.c_float(0.0)
         self._ck(self.L.sparc_gpu_autotune(self.h, int(steps), ctypes.byref(choice), ctypes.byref(ms)))
-        key = "modes_per_cta" if (self.p.precision == "f32" and self.p.nz <= 320) else "threads_per_cta"
+        fused = self.p.nz <= (480 if self.p.option == 4 else 320)
+        key = "modes_per_cta" if (self.p.precision == "f32" and fused) else "threads_per_cta"
         return {key: choice.value, "ms_per_step": ms.value}
 
     def stage(self, rk: int):

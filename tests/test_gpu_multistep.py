@@ -107,3 +107,42 @@ def test_pencil_step_matches_oracle(gpu_lib, oracle_mod, option, nx, ny, nz, nst
     assert nrm(rhs - so) <= (1e-10 if prec == "f64" else 1e-3) * nrm(so)
     if prec == "f64":
         assert nrm(pg - po) <= tol * nrm(po)
+
+
+# the edges of the fused FP32 step's shapes: 3 levels a thread (one and two
+# warps a pencil), 5 levels (one, two and three warps), the smallest box and the largest
+@pytest.mark.parametrize("option,nz", [(4, k) for k in (16, 95, 96, 97, 161, 192, 193, 321, 480)]
+                         + [(17, k) for k in (16, 96, 160, 161, 320)])
+def test_fused_step_shapes(gpu_lib, oracle_mod, option, nz, monkeypatch):
+    """The fused FP32 step against the FP64 oracle: the same sums in another
+    order than the per-stage FP32 kernels, so its error is theirs but for the
+    scatter of rounding (a factor 3 allowed, and never held below 1e-6, eight
+    roundings); and bit for bit the same for every number of modes per CTA."""
+    from cases import smooth_state
+    from sparc_gb300.background import polytrope_table
+    from sparc_gb300.solver import Solver
+    pml_n = max(2, min(10, nz // 6))
+    p = small_params(nx=16, ny=1 if option == 17 else 8, nz=nz, option=option, npmlbot=pml_n, npmltop=pml_n,
+                     precision="f32")
+    tab = polytrope_table(nz, z_bot_mm=-25.0 if nz > 100 else -6.0, z_top_mm=1.0)
+    a0, pml0 = smooth_state(p, seed=7)
+    plane = gaussian_plane(p)
+    series = oracle_mod.forward_source(p, 64) * 1e3
+    o = oracle_mod.Oracle(p, tab)
+    o.set_state(a0, pml0)
+    o.set_source(1, plane[None], series)
+    o.step(3)
+    ao = o.state()[0]
+    out = {}
+    for env, v in [("SPARC_FP32_PER_STAGE", "1")] + [("SPARC_FUSED_MODES", m) for m in "248"]:
+        with monkeypatch.context() as mp:
+            mp.setenv(env, v)
+            with Solver(p, tab) as g:
+                g.set_state(a0, pml0)
+                g.set_source_series(plane, series)
+                g.step(3)
+                out[v] = g.state()
+    err = {v: np.linalg.norm(out[v][0] - ao) / np.linalg.norm(ao) for v in out}
+    assert err["4"] <= max(3 * err["1"], 1e-6)
+    for v in "28":
+        assert np.array_equal(out[v][0], out["4"][0]) and np.array_equal(out[v][1], out["4"][1])
