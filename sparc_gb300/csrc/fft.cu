@@ -2,7 +2,8 @@
 // r2c half-spectrum state (the FFTW plans of initialize.f90:323-337 and
 // damping.f90:46-58 are the reference's counterpart; cuFFT is not used): the
 // register transforms of lines.cuh for 16 to 1024 points, shared-memory
-// Stockham radix-2 FFTs for 4 and 8.
+// Stockham radix-2 FFTs for 4 and 8; FP32 rows of a 2-D grid go through
+// rows2d_f32.cu.
 //
 //   phys -> spec : rows_r2c   (two real rows packed as one complex FFT along x,
 //                              split by Hermitian symmetry, scaled 1/(nx*ny))
@@ -126,9 +127,12 @@ __global__ void spec_mul_kernel(typename CplxOf<T>::type* spec, const T* __restr
 // there is one)
 // rows of nx reals -> rows of H complex (the forward row pass of fft_phys_to_spec)
 template <typename T>
-static void rows_forward(const T* phys, typename CplxOf<T>::type* dst, int nx, long long nrows, T scale,
+static void rows_forward(const T* phys, typename CplxOf<T>::type* dst, int nx, int ny, long long nrows, T scale,
                          const double* tw_x, cudaStream_t s) {
     typedef typename CplxOf<T>::type CT;
+    if constexpr (sizeof(T) == 4) {
+        if (ny == 1) return rows2d_r2c({{phys}, {dst}, 1, 0, 0}, 1, nx, nrows, scale, nullptr, tw_x, {}, s);
+    }
     if (line_ok(nx)) {
         line_r2c<T>({{phys}, {dst}, 1, 0, 0}, 1, nx, nrows, scale, tw_x, {}, s);
         return;
@@ -146,7 +150,7 @@ void fft_phys_to_spec(const T* phys, typename CplxOf<T>::type* spec, typename Cp
     const long long nrows = (long long)ny * nplanes;
     CT* dst = (ny == 1) ? spec : tmp;
     const T scale = (T)(1.0 / ((double)nx * ny));
-    rows_forward<T>(phys, dst, nx, nrows, scale, tw_x, s);
+    rows_forward<T>(phys, dst, nx, ny, nrows, scale, tw_x, s);
     if (ny > 1 && line_ok(ny)) {
         line_cols<T>(tmp, spec, H, ny, nplanes, nplanes, 0LL, -1, mul, tw_y, s);
         return;
@@ -169,6 +173,9 @@ template <typename T>
 static void rows_inverse(const typename CplxOf<T>::type* src, T* phys, int nx, int ny, long long nrows,
                          int rppg, long long rgs, const double* tw_x, cudaStream_t s) {
     typedef typename CplxOf<T>::type CT;
+    if constexpr (sizeof(T) == 4) {
+        if (ny == 1) return rows2d_c2r({{src}, {phys}, 1, 0, 0}, 1, nx, nrows, rppg, rgs, tw_x, {}, s);
+    }
     if (line_ok(nx)) {
         line_c2r<T>({{src}, {phys}, 1, 0, 0}, 1, nx, ny, nrows, rppg, rgs, tw_x, {}, s);
         return;
@@ -218,7 +225,7 @@ int fft_filter_phys(const T* phys, T* out, typename CplxOf<T>::type* spec, typen
         return ny > 1 ? 5 : 3;
     }
     const long long nrows = (long long)ny * nplanes;
-    rows_forward<T>(phys, tmp, nx, nrows, (T)(1.0 / ((double)nx * ny)), tw_x, s);
+    rows_forward<T>(phys, tmp, nx, ny, nrows, (T)(1.0 / ((double)nx * ny)), tw_x, s);
     line_cols_filter<T>({{tmp}, {tmp}, 1, 0, 0}, 1, nx / 2 + 1, ny, nplanes, mul, tw_y, {}, s);
     rows_inverse<T>(tmp, out, nx, ny, nrows, nplanes, 0LL, tw_x, s);
     return 3;

@@ -74,6 +74,16 @@ template <typename T>
 void line_cols_filter(const LineList<typename CplxOf<T>::type, typename CplxOf<T>::type>& L, int nsrc, int H, int ny,
                       long long nplanes, const T* mul, const double* tw, const LineGate& gate, cudaStream_t s);
 
+// The FP32 2-D forms' row transforms (rows2d_f32.cu), any nx: d/dx; rows of nx
+// reals -> rows of nx/2+1 complex, scaled, times mul[k] if given; its inverse, row
+// r at (r / ppg) gstride + (r % ppg) (nx/2+1)
+void rows2d_deriv(const LineList<float, float>& L, int nsrc, int nx, long long nrows, const float* mul, const double* tw,
+                  cudaStream_t s);
+void rows2d_r2c(const LineList<float, float2>& L, int nsrc, int nx, long long nrows, float scale, const float* mul,
+                const double* tw, const LineGate& gate, cudaStream_t s);
+void rows2d_c2r(const LineList<float2, float>& L, int nsrc, int nx, long long nrows, int ppg, long long gstride,
+                const double* tw, const LineGate& gate, cudaStream_t s);
+
 // offset of input plane p when planes come in groups of ppg, group g starting
 // at g * gstride (complex elements); pe = elements per plane
 __device__ __forceinline__ long long grp_off(long long p, int ppg, long long gstride, long long pe) {

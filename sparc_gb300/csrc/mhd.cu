@@ -222,6 +222,14 @@ int ddz_launch(sparc_ctx* c, const T* in, T* out, int bc) { return mhd_ddz<T>(c,
 template <typename T> int mhd_ddx(sparc_ctx* c, const LineList<T, T>& L, int nsrc) {
     const int nx = c->P.nx;
     const long long nrows = (long long)c->nz * c->P.ny;
+    if constexpr (sizeof(T) == 4) {
+        if (c->P.option == 18) {
+            rows2d_deriv(L, nsrc, nx, nrows, (const float*)c->mhd->rx, c->tw_x, c->stream);
+            c->launches++;
+            CKL();
+            return SPARC_OK;
+        }
+    }
     if (line_ok(nx)) {
         line_rows<T>(L, nsrc, nx, nrows, line_mul<T>((const T*)c->mhd->rx), c->tw_x, {}, c->stream);
         c->launches++;
@@ -262,6 +270,7 @@ int mhd_create(sparc_ctx* c) {
     MhdState& m = *c->mhd;
     const size_t es = esz(c);
     int rc;
+    m.rows2d_z = c->f32 && c->P.option == 18 && rows2d_ddz_ok(c->nz);
     if ((rc = dalloc(c, &m.bg, (size_t)MB_COUNT * c->N * es))) return rc;
     CK(cudaMemsetAsync(m.bg, 0, (size_t)MB_COUNT * c->N * es, c->stream));   // 2-D leaves the y rows at 0
     if ((rc = dalloc(c, &m.pab, (size_t)2 * std::max(c->nzpml, 1) * c->NP * es))) return rc;

@@ -40,6 +40,7 @@ struct MhdState {
     void* spec = nullptr;      // [S][3] spectral fields (nz*M complex T): damping / filter transforms
     void* src = nullptr;       // [S][NP] T: a LAGRANGE_INTERP source interpolated to the step
     bool have_bg = false;
+    bool rows2d_z = false;     // FP32 option 18: d/dz through rows2d_ddz
     // sensitivity kernels of the 2-D form (kernels.f90:99-133, 337-453)
     void* kbox = nullptr;      // [N] T: B_x of kernel mode, -ddzkern(psi, 0) / dimb
     void* kcby = nullptr;      // [N] T: (curl B0)_y of kernel mode (CURL_KERN)
@@ -65,5 +66,9 @@ struct ZCodes { int bc[LINE_FIELDS]; };
 template <typename T>
 int mhd_ddz(sparc_ctx* c, const LineList<T, T>& L, const ZCodes& codes, int nsrc, const T* topsrc = nullptr,
             T topscale = (T)0);
+// d/dz of the FP32 2-D form (rows2d_f32.cu); rows2d_ddz_ok: nz fits its shared memory
+bool rows2d_ddz_ok(int nz);
+void rows2d_ddz(const LineList<float, float>& L, const ZCodes& codes, int nsrc, const float* zt, const Compact<float>& cc,
+                long long npix, int nz, const float* topsrc, float topscale, cudaStream_t s);
 // nsteps steps on the context's stream; the context's time is the caller's to advance
 int mhd_enqueue(sparc_ctx* c, int nsteps);

@@ -188,7 +188,7 @@ __device__ __forceinline__ void point2(const StepArgs<T>& A, T* w, const T* __re
             rvz = rvz - sp * vz;
         }
     } else {
-        rvx = ri * (-gpx + cby * boz) + ri * (cboy * bz);
+        rvx = fma(ri, -gpx + cby * boz, ri * (cboy * bz));      // one rounding order (rows2d_f32.cu)
         rvz = ri * (-gpz + (-cby * box)) + ri * (-cboy * bx);
     }
     rvz = rvz - ri * r * __ldg(&A.g[k]);
@@ -498,6 +498,27 @@ int filter_fields(sparc_ctx* c, const LineList<T, T>& L, int nsrc, int row, cons
     MhdState& m = *c->mhd;
     const int nx = c->P.nx, ny = c->P.ny, nz = c->nz;
     const long long nrows = (long long)ny * nz;
+    if constexpr (sizeof(T) == 4) {
+        if (ny == 1) {
+            for (int i0 = 0; i0 < L.n; i0 += 3) {         // m.spec holds three fields of a source
+                LineList<float, float2> f;
+                LineList<float2, float> h;
+                f.n = h.n = std::min(3, L.n - i0);
+                for (int i = 0; i < f.n; ++i) {
+                    float2* sp = (float2*)m.spec + (size_t)i * c->fs;
+                    f.in[i] = L.in[i0 + i]; f.out[i] = sp;
+                    h.in[i] = sp; h.out[i] = L.out[i0 + i];
+                }
+                f.in_ss = L.in_ss; h.out_ss = L.out_ss;
+                f.out_ss = h.in_ss = 3 * c->fs;
+                rows2d_r2c(f, nsrc, nx, nrows, (float)(1.0 / (double)nx), (const float*)c->pt + (size_t)row * c->M, c->tw_x,
+                           gate, c->stream);
+                rows2d_c2r(h, nsrc, nx, nrows, (int)nrows, 0LL, c->tw_x, gate, c->stream);
+                c->launches += 2;
+            }
+            return SPARC_OK;
+        }
+    }
     if (ny == 1) {      // one pass: the packed rows' filter, scaled by 1 / nx
         line_rows<T>(L, nsrc, nx, nrows, line_mul<T>((const T*)m.fx + (row == PT_HF ? nx : 0), true), c->tw_x, gate,
                      c->stream);
@@ -574,7 +595,7 @@ int stage(sparc_ctx* c, const StepArgs<T>& A, int S) {
     } else if constexpr (FORM == 18) {
         // d(xi_x)/dx and d(flux2)/dx, with the damping of v_x, v_z in the same launch where the line transforms cover it
         auto x1 = list({{MW_T0, MW_DX}, {MW_F2, MW_BZ}, {MW_T3, MW_DMX}, {MW_T5, MW_DMZ}});
-        if (A.damp && lines_cover(c)) {
+        if (sizeof(T) == 8 && A.damp && lines_cover(c)) {
             LineMul<T> mul = line_mul<T>((const T*)c->mhd->rx);
             mul.mul[2] = mul.mul[3] = (const T*)c->mhd->fx;
             mul.real = 4 | 8;
@@ -708,6 +729,19 @@ int enqueue_t(sparc_ctx* c, int nsteps) {
 
 template <typename T>
 int mhd_ddz(sparc_ctx* c, const LineList<T, T>& L, const ZCodes& codes, int nsrc, const T* topsrc, T topscale) {
+    if constexpr (sizeof(T) == 4) {
+        if (c->mhd->rows2d_z) {
+            Compact<float> cc;
+            cc.C1 = (float)c->cc64.C1; cc.C2 = (float)c->cc64.C2;
+            for (int i = 0; i < 5; ++i) cc.Cb[i] = (float)c->cc64.Cb[i];
+            for (int i = 0; i < 4; ++i) cc.Cf[i] = (float)c->cc64.Cf[i];
+            cc.alpha2 = (float)c->cc64.alpha2; cc.beta1 = (float)c->cc64.beta1; cc.cnst = (float)c->cc64.cnst;
+            rows2d_ddz(L, codes, nsrc, (const float*)c->zt, cc, c->NP, c->nz, topsrc, topscale, c->stream);
+            c->launches++;
+            CKL();
+            return SPARC_OK;
+        }
+    }
     typedef typename std::conditional<sizeof(T) == 4, float2, T>::type V;
     const long long nv = c->NP / (long long)(sizeof(V) / sizeof(T));
     const int LP = z_pencils(c->nz, nv, L.n * nsrc, c->nsm), nth = LP * z_chunks(c->nz);

@@ -85,3 +85,58 @@ def test_magnetic_step_matches_oracle(gpu_lib, oracle_mod, option, nx, ny, prec,
     ao, _, _ = o.state()
     for f in range(len(ao)):
         assert np.linalg.norm(ag[f] - ao[f]) <= tol * np.linalg.norm(ao[f]), f
+
+
+@pytest.mark.parametrize("nx,nz", [(8, 17), (16, 24), (64, 17), (64, 41), (256, 33), (256, 100), (32, 300), (16, 720)])
+def test_fp32_sheet_step_matches_oracle(gpu_lib, oracle_mod, nx, nz):
+    """One FP32 step of option 18, whose rows and z derivatives have kernels of
+    their own: rows of 64 and 256 points and other sizes, odd row counts, chunks
+    of the z solve that are empty (nz = 17), uneven and whole, and boxes above
+    its limit (720): <= 1e-4 relative L2 per field, as the flux tube's."""
+    from cases import smooth_state
+    from sparc_gb300.background import flux_sheet_background
+    from sparc_gb300.solver import Solver
+    p = _params(nx, 1, nz, option=18, precision="f32", xlength=200e8)
+    tab = table_for(p)
+    bg = flux_sheet_background(p, tab, z_fade_mm=-1.0)
+    a0, pml0 = smooth_state(p, seed=8, npv=6)
+    a0, pml0 = a0 * 1e-3, pml0 * 1e-3
+    o = oracle_mod.Oracle(p, tab)
+    with Solver(p, tab) as g:
+        g.set_mhd2d_background(*bg)
+        o.set_mhd2d(*bg)
+        for s in (g, o):
+            s.set_state(a0, pml0)
+            s.step(1)
+        ag, _ = g.state()
+    ao, _, _ = o.state()
+    for f in range(len(ao)):
+        assert np.linalg.norm(ag[f] - ao[f]) <= 1e-4 * np.linalg.norm(ao[f]), f
+
+
+@pytest.mark.parametrize("nx", [32, 64])
+def test_fp32_sheet_filter_follows_the_slots(gpu_lib, nx):
+    """Option 18, FP32, two slots on different clocks through the horizontal
+    filter's steps: 40 steps of one call equal 40 calls, bit for bit, and a slot
+    equals the same slot run alone."""
+    from cases import smooth_state
+    from sparc_gb300.background import flux_sheet_background
+    from sparc_gb300.solver import Solver
+    out = []
+    for nsrc, calls in ((2, 40), (2, 1), (1, 1)):
+        p = _params(nx, 1, 41, option=18, precision="f32", xlength=400e8, nsrc=nsrc)
+        tab = table_for(p)
+        a0, pml0 = smooth_state(p, seed=9, npv=6)
+        with Solver(p, tab) as g:
+            g.set_mhd2d_background(*flux_sheet_background(p, tab, z_fade_mm=-1.0))
+            for k in range(nsrc):
+                g.set_state(a0 * 1e-3, pml0 * 1e-3, slot=k)
+            if nsrc == 2:
+                g.step(7)
+                g.slot_reset(0)
+                g.set_state(a0 * 1e-3, pml0 * 1e-3, slot=0)
+            for _ in range(calls):
+                g.step(40 // calls)
+            out.append(g.state(0))
+    for b in out[1:]:
+        assert np.array_equal(out[0][0], b[0]) and np.array_equal(out[0][1], b[1])
