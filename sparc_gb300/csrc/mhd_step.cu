@@ -457,6 +457,9 @@ __global__ void __launch_bounds__(Z_THREADS, 2) update_kernel(T* __restrict__ a,
         if (j == 0 || j == nz - 1) v = V(0);
         else if (j >= nz - 5) v = hf * (V(1) + V(-1));
         else if (j <= 4) v = mode == 0 ? hf * (V(1) + V(-1)) : V(0);
+        else if (sizeof(T) == 4 && mode == 0)      // the field's value last: rounds once at its size (as fused.cu)
+            v = V(0) + ((c0 - (T)1) * V(0) + h1 * (V(-1) + V(1)) + h2 * (V(-2) + V(2)) + h3 * (V(-3) + V(3)) +
+                        h4 * (V(-4) + V(4)) + h5 * (V(-5) + V(5)));
         else v = c0 * V(0) + h1 * (V(-1) + V(1)) + h2 * (V(-2) + V(2)) + h3 * (V(-3) + V(3)) + h4 * (V(-4) + V(4)) +
                  h5 * (V(-5) + V(5));
         a[o + (long long)j * npix] = v;
