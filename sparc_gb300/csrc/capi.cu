@@ -9,6 +9,7 @@
 #include <string>
 #include <vector>
 #include <algorithm>
+#include <unistd.h>
 
 #include "ctx.cuh"
 #include "zsolve.cuh"
@@ -989,6 +990,17 @@ static int from_spec_dev(sparc_ctx* c, const void* spec_src, int nplanes) {
     return SPARC_OK;
 }
 
+// Writes a byte of every page of an output buffer about to be copied to.  A page that a
+// fresh allocation has not mapped yet costs the copy to it about 30 us (the copy
+// engine's fault), the CPU 2 us, and the CPU does it while the device still works
+// (state of 256x1x300 FP64, 3.7 MB: 2.0 -> 0.38 ms; 128x128x150, 118 MB: 39 -> 5.9 ms).
+static void map_pages(void* host, size_t bytes) {
+    static const size_t page = (size_t)std::max(sysconf(_SC_PAGESIZE), 4096L);
+    volatile char* p = (volatile char*)host;
+    for (size_t i = 0; i < bytes; i += page) p[i] = 0;
+    if (bytes) p[bytes - 1] = 0;
+}
+
 static int from_spec(sparc_ctx* c, const void* spec_src, double* host_field, int nplanes) {
     // dense planes (MHD) go through phys64 at most nz planes at a time
     const int chunk = c->mhd ? c->nz : nplanes;
@@ -996,6 +1008,7 @@ static int from_spec(sparc_ctx* c, const void* spec_src, double* host_field, int
         const int np = std::min(chunk, nplanes - off);
         int rc = from_spec_dev(c, (const char*)spec_src + (size_t)off * plane_bytes(c), np);
         if (rc) return rc;
+        map_pages(host_field + (long long)off * c->NP, (size_t)c->NP * np * 8);
         CK(cudaMemcpyAsync(host_field + (long long)off * c->NP, c->phys64, (size_t)c->NP * np * 8,
                            cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
@@ -1889,6 +1902,8 @@ int sparc_gpu_kernels(sparc_ctx* c, int src, int sum_slots, double* kc, double* 
     int rc = dalloc(c, (void**)&out, (size_t)3 * c->N * 8);
     if (rc) return rc;
     if ((rc = kernels_finish(c, src, sum_slots, out))) return rc;
+    for (double* h : {kc, krho, hess})
+        if (h) map_pages(h, (size_t)c->N * 8);
     if (kc) CK(cudaMemcpyAsync(kc, out, c->N * 8, cudaMemcpyDeviceToHost, c->stream));
     if (krho) CK(cudaMemcpyAsync(krho, out + c->N, c->N * 8, cudaMemcpyDeviceToHost, c->stream));
     if (hess) CK(cudaMemcpyAsync(hess, out + 2 * c->N, c->N * 8, cudaMemcpyDeviceToHost, c->stream));

@@ -159,7 +159,7 @@ class Solver:
     # ---- state ----
     def field(self, f: int, slot: int = 0, k: int = 0) -> np.ndarray:
         shape = (self.p.ny, self.p.nx) if k > 0 else self.shape
-        out = np.zeros(shape)
+        out = np.empty(shape)
         self._ck(self.L.sparc_gpu_get_field(self.h, slot, f, k, _dp(out)))
         return out
 
@@ -188,7 +188,7 @@ class Solver:
         self._ck(self.L.sparc_gpu_set_mhd2d_background(self.h, *[_dp(v) for v in arrs]))
 
     def state(self, slot: int = 0):
-        a = np.zeros((self.nf,) + self.shape)
+        a = np.empty((self.nf,) + self.shape)
         pml = np.zeros((self.npv, self.p.nzpml, self.p.ny, self.p.nx))
         self._ck(self.L.sparc_gpu_get_state(self.h, slot, _dp(a), _dp(pml)))
         return a, pml
@@ -211,7 +211,7 @@ class Solver:
     def records(self, slot: int = 0) -> np.ndarray:
         n = ctypes.c_int()
         self._ck(self.L.sparc_gpu_get_records(self.h, slot, None, ctypes.byref(n)))
-        out = np.zeros((n.value, self.p.ny, self.p.nx))
+        out = np.empty((n.value, self.p.ny, self.p.nx))
         if n.value:
             self._ck(self.L.sparc_gpu_get_records(self.h, slot, _dp(out), ctypes.byref(n)))
         return out
@@ -287,7 +287,7 @@ class Solver:
         self._ck(self.L.sparc_gpu_kernel_accumulate(fwd.h, int(snap), self.h))
 
     def kernels(self, slot: int = 0, sum_slots: bool = False):
-        kc = np.zeros(self.shape); kr = np.zeros(self.shape); hs = np.zeros(self.shape)
+        kc, kr, hs = (np.empty(self.shape) for _ in range(3))
         self._ck(self.L.sparc_gpu_kernels(self.h, slot, int(sum_slots), _dp(kc), _dp(kr), _dp(hs)))
         return kc, kr, hs
 
