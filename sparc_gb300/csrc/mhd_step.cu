@@ -320,7 +320,9 @@ __global__ void rhs8_kernel(const StepArgs<T> A) {
 
 __device__ __forceinline__ double vfma(double s, double v, double a) { return fma(s, v, a); }
 __device__ __forceinline__ float2 vfma(float s, float2 v, float2 a) { return pfma(bc2(s), v, a); }
+__device__ __forceinline__ float vfma(float s, float v, float a) { return fma(s, v, a); }
 __device__ __forceinline__ double vmul(double s, double v) { return s * v; }
+__device__ __forceinline__ float vmul(float s, float v) { return s * v; }
 __device__ __forceinline__ float2 vmul(float s, float2 v) { return pmul(bc2(s), v); }
 __device__ __forceinline__ double vsub(double a, double b) { return a - b; }
 __device__ __forceinline__ float2 vsub(float2 a, float2 b) { return psub(a, b); }
@@ -430,19 +432,23 @@ int z_pencils(int nz, long long nvalues, int nbatch, int nsm) {
 
 // a += dt*scr (step.f90:114) and the z filter of FILTER_VARS_3D / _2D on whole
 // pencils: a CTA's columns of a + dt*scr meet in shared memory, so the field is
-// read once and written once
-template <typename T>
-__global__ void __launch_bounds__(Z_THREADS, 2) update_kernel(T* __restrict__ a, const T* __restrict__ scr, long long FS,
+// read once and written once.  Bound by memory latency: 256x256x300 FP32, six
+// fields, 446 us with one column per thread, 359 with two (floor 202 us)
+template <typename T, typename V>
+__global__ void __launch_bounds__(Z_THREADS, 2) update_kernel(T* __restrict__ a_, const T* __restrict__ scr_, long long FS,
                                                               long long npix, int nz, int nf, int LP, T dt, int mode) {
     extern __shared__ __align__(16) unsigned char smraw[];
-    T* col = (T*)smraw;                           // [nz][LP]
+    V* col = (V*)smraw;                           // [nz][LP]
+    constexpr int VW = sizeof(V) / sizeof(T);
     const int lp = threadIdx.x & (LP - 1), j0 = threadIdx.x / LP * ZCS;
-    const long long m = (long long)blockIdx.x * LP + lp, o = ((long long)blockIdx.z * nf + blockIdx.y) * FS + m;
-    const bool on = m < npix;
+    const long long nv = npix / VW, m = (long long)blockIdx.x * LP + lp, o = ((long long)blockIdx.z * nf + blockIdx.y) * FS;
+    V* a = (V*)(a_ + o) + m;
+    const V* scr = (const V*)(scr_ + o) + m;
+    const bool on = m < nv;
     #pragma unroll
     for (int q = 0; q < ZCS; ++q) {
         const int j = j0 + q;
-        if (j < nz && on) col[j * LP + lp] = a[o + (long long)j * npix] + dt * scr[o + (long long)j * npix];
+        if (j < nz && on) col[j * LP + lp] = vfma(dt, scr[(long long)j * nv], a[(long long)j * nv]);
     }
     __syncthreads();
     if (!on) return;
@@ -452,17 +458,20 @@ __global__ void __launch_bounds__(Z_THREADS, 2) update_kernel(T* __restrict__ a,
     for (int q = 0; q < ZCS; ++q) {
         const int j = j0 + q;
         if (j >= nz) break;
-        auto V = [&](int i) -> T { return col[(j + i) * LP + lp]; };
-        T v;
-        if (j == 0 || j == nz - 1) v = V(0);
-        else if (j >= nz - 5) v = hf * (V(1) + V(-1));
-        else if (j <= 4) v = mode == 0 ? hf * (V(1) + V(-1)) : V(0);
-        else if (sizeof(T) == 4 && mode == 0)      // the field's value last: rounds once at its size (as fused.cu)
-            v = V(0) + ((c0 - (T)1) * V(0) + h1 * (V(-1) + V(1)) + h2 * (V(-2) + V(2)) + h3 * (V(-3) + V(3)) +
-                        h4 * (V(-4) + V(4)) + h5 * (V(-5) + V(5)));
-        else v = c0 * V(0) + h1 * (V(-1) + V(1)) + h2 * (V(-2) + V(2)) + h3 * (V(-3) + V(3)) + h4 * (V(-4) + V(4)) +
-                 h5 * (V(-5) + V(5));
-        a[o + (long long)j * npix] = v;
+        auto W = [&](int i) -> V { return col[(j + i) * LP + lp]; };
+        V v;
+        if (j == 0 || j == nz - 1) v = W(0);
+        else if (j >= nz - 5) v = vmul(hf, W(1) + W(-1));
+        else if (j <= 4) v = mode == 0 ? vmul(hf, W(1) + W(-1)) : W(0);
+        else if constexpr (VW == 2) {      // the field's value last: rounds once at its size (as fused.cu)
+            v = vfma(h1, W(-1) + W(1), vmul(c0 - (T)1, W(0)));
+            v = vfma(h3, W(-3) + W(3), vfma(h2, W(-2) + W(2), v));
+            v = W(0) + vfma(h5, W(-5) + W(5), vfma(h4, W(-4) + W(4), v));
+        } else {
+            v = c0 * W(0) + h1 * (W(-1) + W(1)) + h2 * (W(-2) + W(2)) + h3 * (W(-3) + W(3)) + h4 * (W(-4) + W(4)) +
+                h5 * (W(-5) + W(5));
+        }
+        a[(long long)j * nv] = v;
     }
 }
 
@@ -666,7 +675,13 @@ int enqueue_t(sparc_ctx* c, int nsteps) {
     A.src_ss = c->src_mode == 2 ? c->NP : (long long)c->src_L * c->NP;
     A.series = c->series; A.nseries = c->nseries;
     A.plane = m.plane; A.dw = (const T*)m.dw;
-    const int LP = z_pencils(nz, c->NP, c->nf * S, c->nsm), nth = LP * z_chunks(nz);
+    // update: two neighbouring columns per thread in FP32, but not in 2-D, whose FP32
+    // sums keep their order (rows2d_f32.cu)
+    const int vw = sizeof(T) == 4 && !two_d ? 2 : 1;
+    const long long unv = c->NP / vw;
+    const int LP = z_pencils(nz, unv, c->nf * S, c->nsm), nth = LP * z_chunks(nz);
+    const dim3 ug((unsigned)((unv + LP - 1) / LP), c->nf, S);
+    const size_t usm = (size_t)nz * LP * vw * sizeof(T);
     LineGate gate;
     gate.on = 1;
     gate.clk = A.clk;
@@ -684,9 +699,14 @@ int enqueue_t(sparc_ctx* c, int nsteps) {
             const int rc = two_d ? stage<T, 18>(c, A, S) : (opt == 8 ? stage<T, 8>(c, A, S) : stage<T, 10>(c, A, S));
             if (rc) return rc;
         }
-        update_kernel<T><<<dim3((unsigned)((c->NP + LP - 1) / LP), c->nf, S), nth, (size_t)nz * LP * sizeof(T),
-                           c->stream>>>((T*)c->a, (const T*)c->scr, A.FS, c->NP, nz, c->nf, LP, (T)c->deltat,
-                                        two_d ? 1 : 0);
+        if constexpr (sizeof(T) == 4) {
+            if (!two_d)
+                update_kernel<T, float2><<<ug, nth, usm, c->stream>>>((T*)c->a, (const T*)c->scr, A.FS, c->NP, nz, c->nf, LP,
+                                                                      (T)c->deltat, 0);
+        }
+        if (vw == 1)
+            update_kernel<T, T><<<ug, nth, usm, c->stream>>>((T*)c->a, (const T*)c->scr, A.FS, c->NP, nz, c->nf, LP,
+                                                             (T)c->deltat, two_d ? 1 : 0);
         const long long npv = (long long)S * PV_COUNT * A.nzpml * c->NP;
         pml_update_kernel<T><<<nb256(npv), 256, 0, c->stream>>>((T*)m.pml, (const T*)m.spml, (T)c->deltat, npv);
         c->launches += 2;
