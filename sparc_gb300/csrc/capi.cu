@@ -12,6 +12,7 @@
 #include <unistd.h>
 
 #include "ctx.cuh"
+#include "lines.cuh"
 #include "zsolve.cuh"
 #include "adjsrc.cuh"
 #include "update.cuh"
@@ -1715,8 +1716,17 @@ static int derive_to_phys(sparc_ctx* c, int s0, int G, bool adjoint, T* out, lon
     CT* D = CP<T>(c->ybuf);      // [G][fs] each
     CT* D2 = CP<T>(c->pbuf);
     CT* D3 = CP<T>(c->rbuf);
+    const int nx = c->P.nx, ny = c->P.ny, nz = c->nz, M = c->M;
+    // Whether a launch takes all sources, and the three components of a vector:
+    // where the column passes' intermediate of that stays in L2 (48 MB).  64x64x75,
+    // two sources: a snapshot's 30 launches become 8, 162 -> 71 us; 32x32x50 FP64,
+    // eight sources: 1031 -> 259 us.  A larger one goes one source and field at a
+    // time, so that each intermediate (79 MB in FP32 at 256x256x300) stays in L2
+    // for the row pass right after
+    const size_t field_bytes = (size_t)kernel_group(c->S) * fs * csz(c);
+    const bool batch = ny > 1 && line_ok(nx) && line_ok(ny) && 3 * field_bytes <= (size_t)48 << 20;
     if (!c->gtmp) {
-        int rc = dalloc(c, &c->gtmp, (size_t)kernel_group(c->S) * fs * 2 * esz(c));
+        int rc = dalloc(c, &c->gtmp, (batch ? 3 : 1) * field_bytes);
         if (rc) return rc;
     }
     CT* tmp = CP<T>(c->gtmp);
@@ -1727,17 +1737,36 @@ static int derive_to_phys(sparc_ctx* c, int s0, int G, bool adjoint, T* out, lon
     cc.alpha2 = (T)c->cc64.alpha2; cc.beta1 = (T)c->cc64.beta1; cc.cnst = (T)c->cc64.cnst;
     const T* zt = (const T*)c->zt;
     const T* pt = (const T*)c->pt;
-    const int nx = c->P.nx, ny = c->P.ny, nz = c->nz, M = c->M;
     const bool use_y = ny > 4;
-    // spectral fields of the group -> physical: src_ss = source stride of the
-    // input.  One source per transform: its column-pass intermediate (nz
-    // planes of the half spectrum, 79 MB in FP32 at 256x256x300) stays in L2
-    // for the row pass that reads it right after
+    // spectral fields of the group -> physical: src_ss = source stride of the input
     auto tophys = [&](const CT* spec, long long src_ss, T* dst) {
+        if (batch) {
+            fft_spec_to_phys_g<T>(spec, nz, src_ss, dst, tmp, nx, ny, G * nz, c->tw_x, c->tw_y, c->stream);
+            c->launches += 2;
+            return;
+        }
         for (int g = 0; g < G; ++g)
             fft_spec_to_phys_g<T>(spec + (long long)g * src_ss, nz, 0LL, dst + (long long)g * N, tmp, nx, ny, nz,
                                   c->tw_x, c->tw_y, c->stream);
         c->launches += 2 * G;
+    };
+    // three fields next to each other in the state -> physical, field stride ofs
+    auto tophys3 = [&](const CT* spec, T* dst) {
+        if (!batch) {
+            for (int q = 0; q < 3; ++q) tophys(spec + q * fs, 6 * fs, dst + q * ofs);
+            return;
+        }
+        line_cols<T>(spec, tmp, nx / 2 + 1, ny, 3LL * G * nz, 3 * nz, 6 * fs, 1, nullptr, c->tw_y, c->stream);
+        LineList<CT, T> L;
+        L.n = 3;
+        L.in_ss = 3 * fs;
+        L.out_ss = N;
+        for (int q = 0; q < 3; ++q) {
+            L.in[q] = tmp + q * fs;
+            L.out[q] = dst + q * ofs;
+        }
+        line_c2r<T>(L, G, nx, ny, (long long)ny * nz, nz, 0LL, c->tw_x, {}, c->stream);
+        c->launches += 2;
     };
     // divergence: ddxkern + ddykern + ddzkern(bc=1, filtered)  (COMPUTE_DIV kernels.f90:798-816)
     const int fx = adjoint ? 3 : 0;
@@ -1746,10 +1775,10 @@ static int derive_to_phys(sparc_ctx* c, int s0, int G, bool adjoint, T* out, lon
     c->launches += 2;
     tophys(D, fs, out);
     if (!adjoint) {
-        for (int q = 0; q < 3; ++q) tophys(scr + (3 + q) * fs, 6 * fs, out + (1 + q) * ofs);   // f_acc
-        for (int q = 0; q < 3; ++q) tophys(a + q * fs, 6 * fs, out + (4 + q) * ofs);           // f_xi
+        tophys3(scr + 3 * fs, out + ofs);       // f_acc
+        tophys3(a, out + 4 * ofs);              // f_xi
     } else {
-        for (int q = 0; q < 3; ++q) tophys(a + (3 + q) * fs, 6 * fs, out + (1 + q) * ofs);     // a_v
+        tophys3(a + 3 * fs, out + ofs);         // a_v
         // grad(a_vz * grav) (kernels.f90:299-304)
         launch_spec_scale_z<T>(D2, a + 5 * fs, zt, ZT_GRAW, M, nz, G, fs, 6 * fs, c->stream);
         launch_spec_dxdy<T>(D3, D2, pt, 0, M, nz, G, fs, fs, c->stream);

@@ -146,3 +146,31 @@ def test_fused_step_shapes(gpu_lib, oracle_mod, option, nz, monkeypatch):
     assert err["4"] <= max(3 * err["1"], 1e-6)
     for v in "28":
         assert np.array_equal(out[v][0], out["4"][0]) and np.array_equal(out[v][1], out["4"][1])
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(16, 16, 17), (64, 32, 41), (32, 64, 75)])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_kernels_of_a_batch_equal_single_sources(gpu_lib, nx, ny, nz, prec):
+    """A small grid's snapshot and accumulation transform all sources, and three
+    fields, per launch: the kernels of each slot of a batch are bit for bit those
+    of the same source run alone (batches of 3, and of 9: a full group and a rest)."""
+    from sparc_gb300.solver import Solver
+    def run(nsrc, first):
+        fwd = small_params(nx=nx, ny=ny, nz=nz, npmlbot=4, npmltop=4, precision=prec, nsrc=nsrc)
+        adj = small_params(nx=nx, ny=ny, nz=nz, npmlbot=4, npmltop=4, precision=prec, nsrc=nsrc, compute_forward=False,
+                           compute_adjoint=True)
+        with Solver(fwd, table_for(fwd)) as f, Solver(adj, table_for(adj)) as a:
+            for k in range(nsrc):
+                f.set_state(*random_state(fwd, seed=20 + first + k), slot=k)
+                a.set_state(*random_state(adj, seed=40 + first + k), slot=k)
+            for _ in range(2):
+                f.step(1)
+                a.step(1)
+                f.snapshot(0, 1)
+                a.kernel_accumulate(f, 0)
+            return [a.kernels(k) for k in range(nsrc)]
+    alone = [run(1, k)[0] for k in range(9)]
+    for nsrc in (3, 9):
+        for k, got in enumerate(run(nsrc, 0)):
+            for x, y in zip(got, alone[k]):
+                assert np.array_equal(x, y)
