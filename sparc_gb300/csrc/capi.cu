@@ -552,8 +552,8 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
                         getenv(c->f32 ? "SPARC_FP32_PER_STAGE" : "SPARC_STAGE_LANES") == nullptr &&
                         pencil_count(c->pencil, opt, c->nzpml, (int)cs, 1, c->nsm) > 0 &&
                         pencil_ok(c->nz, c->pencil, bc1, bc2) &&
-                        (c->f32 ? pencil_prepare<float>(c->pencil, opt, c->nzpml)
-                                : pencil_prepare<double>(c->pencil, opt, c->nzpml));
+                        (c->f32 ? pencil_prepare<float>(c->pencil, opt)
+                                : pencil_prepare<double>(c->pencil, opt));
         if (c->use_pencil && (rc = dalloc(c, &c->ptab, pencil_table_size(c->pencil, c->nzpml) * es))) return bail(rc);
         if ((c->use_pencil || c->use_fused) &&
             (rc = dalloc(c, &c->src_plane, (size_t)FUSED_STEPS * c->S * c->M * cs))) return bail(rc);

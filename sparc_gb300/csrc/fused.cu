@@ -800,9 +800,7 @@ namespace {
 template <bool D3, int W, int P, int CH>
 int launch_fused_t(const FusedArgs& A, int nsrc, bool prepare, cudaStream_t s) {
     const size_t sm = (size_t)fused_layout(P, W, CH, A.nzpml).total;
-    if (prepare)
-        return cudaFuncSetAttribute((const void*)fused_step_kernel<D3, W, P, CH>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
+    if (prepare) return allow_shared_memory((const void*)fused_step_kernel<D3, W, P, CH>);
     FusedArgs B = A;
     B.nsrc = nsrc;
     int dev = 0, nsm = 0, occ = 0;

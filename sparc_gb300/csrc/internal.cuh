@@ -277,6 +277,17 @@ __device__ __forceinline__ CT* smem_fft(CT* src, CT* dst, int n, int count, T si
     return src;
 }
 
+// Lets every launch of a kernel take all the shared memory a CTA may have
+// (227 KB less its static part).  The limit belongs to the function, not to a
+// context: set to one context's size, it would refuse the launches of another
+// context on a taller grid.
+inline bool allow_shared_memory(const void* kernel) {
+    cudaFuncAttributes a;
+    return cudaFuncGetAttributes(&a, kernel) == cudaSuccess &&
+           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                227 * 1024 - (int)a.sharedSizeBytes) == cudaSuccess;
+}
+
 // ---- argument blocks ----------------------------------------------------------
 template <typename T> struct StageArgs {
     typedef typename CplxOf<T>::type CT;
@@ -422,7 +433,7 @@ template <typename T> struct PencilArgs {
 };
 PencilShape pencil_shape(int nz, int modes);
 int pencil_count(const PencilShape& sh, int option, int nzpml, int complex_bytes, long long pencils, int nsm);
-template <typename T> int pencil_prepare(const PencilShape& sh, int option, int nzpml);
+template <typename T> int pencil_prepare(const PencilShape& sh, int option);
 template <typename T> void launch_pencil(const PencilArgs<T>& A, int ch, cudaStream_t s);
 // each step's source plane of a launch of nsteps steps (fused.cu), LAGRANGE_INTERP
 template <typename T>

@@ -651,14 +651,8 @@ int pencil_count(const PencilShape& sh, int option, int nzpml, int complex_bytes
 }
 
 template <typename T>
-int pencil_prepare(const PencilShape& sh, int option, int nzpml) {
-    size_t smem = 0;
-    for (int P = std::max(1, 128 / (32 * sh.W)); P >= 1; P /= 2) {
-        const size_t b = pencil_bytes(sh, option, P, nzpml, 2 * sizeof(T));
-        if (b <= 227 * 1024) smem = std::max(smem, b);
-    }
-    return cudaFuncSetAttribute(kernel_of<T>(option, sh.ch), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-           cudaSuccess;
+int pencil_prepare(const PencilShape& sh, int option) {
+    return allow_shared_memory(kernel_of<T>(option, sh.ch));
 }
 
 template <typename T>
@@ -669,7 +663,7 @@ void launch_pencil(const PencilArgs<T>& A, int ch, cudaStream_t s) {
     cudaLaunchKernel(kernel_of<T>(A.option, ch), dim3((unsigned)ctas), dim3(A.pencils * 32 * A.W), args, smem, s);
 }
 
-template int pencil_prepare<double>(const PencilShape&, int, int);
-template int pencil_prepare<float>(const PencilShape&, int, int);
+template int pencil_prepare<double>(const PencilShape&, int);
+template int pencil_prepare<float>(const PencilShape&, int);
 template void launch_pencil<double>(const PencilArgs<double>&, int, cudaStream_t);
 template void launch_pencil<float>(const PencilArgs<float>&, int, cudaStream_t);

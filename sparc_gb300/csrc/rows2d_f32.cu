@@ -461,9 +461,7 @@ void rows2d_c2r(const LineList<float2, float>& L, int nsrc, int nx, long long nr
 
 // pencils that fit the kernel's shared memory (about 700 levels; taller ones go through mhd_ddz's own solver)
 bool rows2d_ddz_ok(int nz) {
-    const size_t sm = chunk_bytes(nz);
-    return sm <= 200 * 1024 &&
-           cudaFuncSetAttribute((const void*)ddz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) == cudaSuccess;
+    return chunk_bytes(nz) <= 200 * 1024 && allow_shared_memory((const void*)ddz_kernel);
 }
 
 void rows2d_ddz(const LineList<float, float>& L, const ZCodes& codes, int nsrc, const float* zt, const Compact<float>& cc,
