@@ -219,9 +219,12 @@ def timed_region(fwd, adj, steps, cad):
     return e0.elapsed_time(e1), launches
 
 
-def step_kernel_time(solver, n=15, reps=2):
-    """Average duration of one time-step launch (the fused FP32 step kernel is
-    the only kernel of a step), CUDA events on the launching stream."""
+FUSED_LAUNCH_STEPS = 15      # time steps of a fused launch between two kernel snapshots (16 at most)
+
+
+def step_kernel_time(solver, n=FUSED_LAUNCH_STEPS, reps=2):
+    """Average duration of one time step (n of them are one launch of the fused
+    FP32 step kernel), CUDA events on the launching stream."""
     import torch
     s = torch.cuda.ExternalStream(solver.stream_ptr)
     solver.sync()
@@ -255,7 +258,7 @@ def issue_roofline(winst, launch_ms, clocks, sm_count):
     return {"warp_inst_per_launch": winst, "achieved_ginst_s": ach / 1e9, "peak_ginst_s": peak / 1e9,
             "frac": ach / peak, "sm_mhz": mhz, "sms": sm_count,
             "source": "smsp__inst_executed.sum of one ncu capture of a single-source launch at this grid, "
-                      "times nsrc"}
+                      "per step, times nsrc"}
 
 
 def serving_section(precision: str, n: int, compress: float, rate: float = 4.0, seed: int = 0,
@@ -813,11 +816,12 @@ def main():
     value = 2 * N * S * K * ws / (ms * 1e-3) / 1e6
     # roofline of the dominant kernel (the fused FP32 step): its own
     # compulsory bytes per launch (12 field accesses, the PML planes and the
-    # source plane of every source) over its average launch time
-    own = bytes_model.fused_step_alg_bytes(p32)
-    achieved = own / (st_ms * 1e-3) / 1e9
+    # source planes of every source) over its average launch time
+    launch_ms = st_ms * FUSED_LAUNCH_STEPS
+    own = bytes_model.fused_step_alg_bytes(p32, steps=FUSED_LAUNCH_STEPS)
+    achieved = own / (launch_ms * 1e-3) / 1e9
     traffic = bytes_model.fused_traffic_per_launch(p32)
-    winst = bytes_model.fused_warp_inst_per_launch(p32)
+    winst = bytes_model.fused_warp_inst_per_launch(p32, FUSED_LAUNCH_STEPS)
     # the per-stage schedule's credit (653.3 B per grid-point-step), kept
     # apart: it counts bytes this kernel does not move
     bpps = bytes_model.reference_schedule_bytes_per_point_step("f32")
@@ -894,18 +898,20 @@ def main():
         "clocks": clocks,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                      "frac": achieved / hbm_peak, "traffic": traffic,
-                     "kernel": "fused_step_kernel (FP32, one launch per time step of all sources)",
-                     "avg_launch_ms": st_ms, "alg_bytes_per_launch": own,
-                     "alg_bytes_per_point_step": own / (N * S),
-                     "alg_what": "compulsory bytes of the fused step: read and write a (12 spectral field "
+                     "kernel": "fused_step_kernel (FP32, one launch per "
+                               f"{FUSED_LAUNCH_STEPS} time steps of all sources)",
+                     "avg_launch_ms": launch_ms, "steps_per_launch": FUSED_LAUNCH_STEPS, "ms_per_time_step": st_ms,
+                     "alg_bytes_per_launch": own,
+                     "alg_bytes_per_point_step": own / (N * S * FUSED_LAUNCH_STEPS),
+                     "alg_what": "compulsory bytes of a fused launch: read and write a (12 spectral field "
                                  "accesses), the two PML auxiliaries on their planes (read and write), one "
-                                 "source plane, per source",
+                                 "source plane per step, per source",
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of a "
                                        "single-source launch at this grid, times nsrc (a scaled constant, not "
                                        "measured in this run)" if traffic else None,
-                     "issue": issue_roofline(winst, st_ms, clocks, sm_count),
+                     "issue": issue_roofline(winst, launch_ms, clocks, sm_count),
                      "schedule_credit": {
-                         "bytes_per_point_step": bpps, "bytes_per_launch": bpps * N * S,
+                         "bytes_per_point_step": bpps, "bytes_per_step": bpps * N * S,
                          "achieved_gbs": bpps * N * S / (st_ms * 1e-3) / 1e9,
                          "frac": bpps * N * S / (st_ms * 1e-3) / 1e9 / hbm_peak,
                          "what": "the compulsory bytes of the minimal per-stage schedule of the reference's "

@@ -18,12 +18,12 @@ tridiagonal intermediates y, p', rho' round-tripping through global memory):
 The difference (10 accesses per stage) is the traffic that an on-chip schedule
 removes.
 
-The fused FP32 step (fused.cu) keeps a pencil's state on chip for the whole
-step: per step it reads a (6 fields) and writes a (6 fields), plus the PML
-planes (2 fields on nzpml planes, read + write) and one source plane per
-source; the stage right-hand side scr (6 fields) is written only on steps whose
-outputs need it.  Its algorithmic and implemented counts coincide: 12 field
-accesses per step, against 102 for the per-stage schedule.
+The fused FP32 step (fused.cu) keeps a pencil's state on chip for all the steps
+of a launch: per launch it reads a (6 fields) and writes a (6 fields), plus the
+PML planes (2 fields on nzpml planes, read + write) and one source plane per
+source and step; the stage right-hand side scr (6 fields) is written only on
+steps whose outputs need it.  Its algorithmic and implemented counts coincide:
+12 field accesses per launch, against 102 per step for the per-stage schedule.
 """
 from __future__ import annotations
 
@@ -122,26 +122,27 @@ def mhd_schedule_bytes_per_point_step(precision: str) -> float:
 FUSED_STEP = 12
 
 
-def fused_step_alg_bytes(p, write_scr: bool = False) -> int:
-    """Bytes of one fused-step launch (all sources)."""
+def fused_step_alg_bytes(p, write_scr: bool = False, steps: int = 1) -> int:
+    """Bytes of one fused launch of `steps` time steps (all sources): the state
+    once, a source plane per step."""
     f = field_bytes(p)
     pf = pml_field_bytes(p)
     plane = (p.nx // 2 + 1) * p.ny * complex_bytes(p.precision) * p.nsrc
-    return (FUSED_STEP + (6 if write_scr else 0)) * f + 4 * pf + plane
+    return (FUSED_STEP + (6 if write_scr else 0)) * f + 4 * pf + steps * plane
 
 
-#: DRAM traffic (read + write) of one fused-step launch per source:
-#: dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of a
-#: single-source forward step (no scr written) at 256x256x300 FP32.  Traffic
-#: grows in proportion to the number of sources, so a batched launch is
-#: credited with this figure times nsrc; it is a scaled constant, not a
-#: measurement of the run that reports it.
-MEASURED_FUSED_TRAFFIC_PER_SOURCE = {(256, 256, 300, "f32"): 920.0e6}
+#: DRAM traffic (read + write) of one fused launch per source, whatever its
+#: number of steps: dram__bytes_read.sum + dram__bytes_write.sum of one ncu
+#: capture of a single-source forward launch (16 steps, no scr written) at
+#: 256x256x300 FP32.  Traffic grows in proportion to the number of sources, so
+#: a batched launch is credited with this figure times nsrc; it is a scaled
+#: constant, not a measurement of the run that reports it.
+MEASURED_FUSED_TRAFFIC_PER_SOURCE = {(256, 256, 300, "f32"): 919.2e6}
 
-#: Warp instructions executed by one fused-step launch per source
-#: (smsp__inst_executed.sum of the same ncu capture), for the issue-side
-#: roofline: a launch of nsrc sources issues this many times nsrc.
-MEASURED_FUSED_WARP_INST_PER_SOURCE = {(256, 256, 300, "f32"): 424.3e6}
+#: Warp instructions executed per source and time step of a fused launch
+#: (smsp__inst_executed.sum of the same ncu capture / 16), for the issue-side
+#: roofline: a launch of nsrc sources issues this many times nsrc a step.
+MEASURED_FUSED_WARP_INST_PER_SOURCE = {(256, 256, 300, "f32"): 349.5e6}
 
 
 def fused_traffic_per_launch(p):
@@ -149,6 +150,6 @@ def fused_traffic_per_launch(p):
     return None if v is None else v * p.nsrc
 
 
-def fused_warp_inst_per_launch(p):
+def fused_warp_inst_per_launch(p, steps: int):
     v = MEASURED_FUSED_WARP_INST_PER_SOURCE.get((p.nx, p.ny, p.nz, p.precision))
-    return None if v is None else v * p.nsrc
+    return None if v is None else v * p.nsrc * steps

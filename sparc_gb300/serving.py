@@ -133,9 +133,8 @@ class Pool:
         """Queue nsteps more steps (one step on the flux tube), unless two
         such chunks are still queued: the GPU queues stay short, so the
         streams' priorities decide the order of the pools' work.  A flux-tube
-        step is hundreds of separate launches (its per-slot filter schedule
-        keeps it out of graphs); queuing one at a time keeps the host from
-        blocking on a full launch queue while cheap pools wait.  Returns
+        step is about a hundred kernels of a graph and takes milliseconds;
+        queuing one at a time keeps cheap pools from waiting behind it.  Returns
         whether steps were queued."""
         import torch
         if not self.busy:
