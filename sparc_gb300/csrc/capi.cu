@@ -1101,7 +1101,10 @@ int sparc_gpu_set_source(sparc_ctx* c, int src, int mode, const double* planes, 
         c->src_set[src] = 0;
         bool any = false;
         for (int s : c->src_set) any = any || s;
-        if (!any) c->src_mode = 0;
+        if (!any && c->src_mode != 0) {
+            c->src_mode = 0;
+            c->epoch++;                       // captured steps hold the mode
+        }
         return SPARC_OK;
     }
     if (mode != SPARC_SRC_SERIES && mode != SPARC_SRC_LAGRANGE) return fail(c, SPARC_EINVAL, "bad source mode");
