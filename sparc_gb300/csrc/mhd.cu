@@ -35,12 +35,17 @@ __device__ __forceinline__ typename CplxOf<T>::type imul_c(T k, typename CplxOf<
     return r;
 }
 
-// d/dx of nrows rows of nx reals (rows r = plane*ny + y, dense), two rows per CTA
+// d/dx of nrows rows of nx reals (rows r = plane*ny + y, dense), two rows per CTA;
+// every field (grid.y) and source (grid.z) of a list in one launch, since a grid
+// this small is bound by its launches (option 10, 8x8x41, two sources, a step
+// with a launch each 1.43 ms in FP32 and 1.87 in FP64, so 0.87 and 1.19)
 template <typename T>
-__global__ void rowderiv_kernel(const T* __restrict__ in, T* __restrict__ out, int nx, long long nrows,
-                                const T* __restrict__ rx, const double* __restrict__ tw) {
+__global__ void rowderiv_kernel(const LineList<T, T> L, int nx, long long nrows, const T* __restrict__ rx,
+                                const double* __restrict__ tw) {
     typedef typename CplxOf<T>::type CT;
     extern __shared__ __align__(16) unsigned char smraw[];
+    const T* in = L.in[blockIdx.y] + blockIdx.z * L.in_ss;
+    T* out = L.out[blockIdx.y] + blockIdx.z * L.out_ss;
     CT* b0 = (CT*)smraw;
     CT* b1 = b0 + nx;
     const long long r0 = 2LL * blockIdx.x, r1 = r0 + 1;
@@ -62,12 +67,15 @@ __global__ void rowderiv_kernel(const T* __restrict__ in, T* __restrict__ out, i
     }
 }
 
-// d/dy of nplanes dense (ny, nx) planes: W complex columns (2W real x) per CTA
+// d/dy of nplanes dense (ny, nx) planes: W complex columns (2W real x) per CTA;
+// fields and sources as rowderiv_kernel
 template <typename T>
-__global__ void colderiv_kernel(const T* __restrict__ in, T* __restrict__ out, int nx, int ny, int W,
-                                const T* __restrict__ ry, const double* __restrict__ tw) {
+__global__ void colderiv_kernel(const LineList<T, T> L, int nx, int ny, int W, const T* __restrict__ ry,
+                                const double* __restrict__ tw) {
     typedef typename CplxOf<T>::type CT;
     extern __shared__ __align__(16) unsigned char smraw[];
+    const T* in = L.in[blockIdx.y] + blockIdx.z * L.in_ss;
+    T* out = L.out[blockIdx.y] + blockIdx.z * L.out_ss;
     CT* b0 = (CT*)smraw;
     CT* b1 = b0 + (long long)W * ny;
     const int ntile = (nx / 2) / W;
@@ -235,10 +243,9 @@ template <typename T> int mhd_ddx(sparc_ctx* c, const LineList<T, T>& L, int nsr
         c->launches++;
     } else {
         const size_t sm = 2 * (size_t)nx * sizeof(typename CplxOf<T>::type);
-        for (int s = 0; s < nsrc; ++s)
-            for (int i = 0; i < L.n; ++i, c->launches++)
-                rowderiv_kernel<T><<<(unsigned)((nrows + 1) / 2), 32, sm, c->stream>>>(
-                    L.in[i] + s * L.in_ss, L.out[i] + s * L.out_ss, nx, nrows, (const T*)c->mhd->rx, c->tw_x);
+        rowderiv_kernel<T><<<dim3((unsigned)((nrows + 1) / 2), L.n, nsrc), 32, sm, c->stream>>>(
+            L, nx, nrows, (const T*)c->mhd->rx, c->tw_x);
+        c->launches++;
     }
     CKL();
     return SPARC_OK;
@@ -252,10 +259,9 @@ template <typename T> int mhd_ddy(sparc_ctx* c, const LineList<T, T>& L, int nsr
     } else {
         const int W = std::max(1, std::min(nx / 2, 1024 / ny));
         const size_t sm = 2 * (size_t)W * ny * sizeof(typename CplxOf<T>::type);
-        for (int s = 0; s < nsrc; ++s)
-            for (int i = 0; i < L.n; ++i, c->launches++)
-                colderiv_kernel<T><<<(unsigned)((long long)c->nz * ((nx / 2) / W)), 256, sm, c->stream>>>(
-                    L.in[i] + s * L.in_ss, L.out[i] + s * L.out_ss, nx, ny, W, (const T*)c->mhd->ry, c->tw_y);
+        colderiv_kernel<T><<<dim3((unsigned)((long long)c->nz * ((nx / 2) / W)), L.n, nsrc), 256, sm, c->stream>>>(
+            L, nx, ny, W, (const T*)c->mhd->ry, c->tw_y);
+        c->launches++;
     }
     CKL();
     return SPARC_OK;

@@ -101,3 +101,31 @@ def test_z_derivatives_at_the_edges_of_the_chunks(gpu_lib, oracle_mod, option, p
         assert nrm(ag[f] - ao[f]) <= tol * nrm(ao[f]), f
     assert nrm(rg - ro) <= rtol * nrm(ro)
     assert nrm(pg - po) <= rtol * nrm(po)
+
+
+@pytest.mark.parametrize("option,nx,ny", [(8, 8, 8), (10, 8, 8), (10, 4, 16), (10, 16, 4), (8, 4, 4), (18, 8, 1)])
+@pytest.mark.parametrize("prec,tol", [("f64", 1e-10), ("f32", 1e-4)])
+def test_grids_below_the_line_transforms(gpu_lib, oracle_mod, option, nx, ny, prec, tol):
+    """Three steps of two sources on grids of 4 or 8 points a side, whose x and y
+    derivatives take all fields and sources of a group per launch: each slot
+    against the oracle, as the other magnetic steps."""
+    from sparc_gb300.solver import Solver
+    p = _params(option, prec, nz=41, nx=nx, ny=ny, nsrc=2)
+    tab = table_for(p)
+    bg = _background(p, tab)
+    with Solver(p, tab) as g:
+        (g.set_mhd2d_background if option == 18 else g.set_mhd_background)(*bg)
+        want = []
+        for k in range(2):
+            a0, pml0 = smooth_state(p, seed=50 + k, scale=1e-6, nf=g.nf, npv=6)
+            o = oracle_mod.Oracle(p, tab)
+            (o.set_mhd2d if option == 18 else o.set_mhd)(*bg)
+            o.set_state(a0, pml0)
+            g.set_state(a0, pml0, slot=k)
+            o.step(3)
+            want.append(o.state()[0])
+        g.step(3)
+        for k in range(2):
+            got = g.state(k)[0]
+            for f in range(g.nf):
+                assert np.linalg.norm(got[f] - want[k][f]) <= tol * np.linalg.norm(want[k][f]), (k, f)
