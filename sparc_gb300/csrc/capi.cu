@@ -200,10 +200,26 @@ double pencil_omitted(const FusedRows& r, int ch, int nz) {
 
 // Whether the carries of pencil.cu are exact to 2^-60 for the two boundary codes of a form
 bool pencil_ok(int nz, const PencilShape& sh, int bc1, int bc2) {
-    const int nzp = 32 * sh.W * sh.ch;
+    const int nzp = sh.tp * sh.ch;
     for (int b : {bc1, bc2})
         if (pencil_omitted(fused_rows(nz, nzp, tri_for(nz, b), sh.ch), sh.ch, nz) > 8.6736173798840355e-19) return false;
     return true;
+}
+
+// Whether the FP64 per-stage kernels are faster than pencil.cu on a grid.  They walk
+// a pencil's levels on one or a few threads, through HBM: bound by latency on few
+// pencils, and without a price for lanes that hold no level.  Measured per step of
+// option 4, per stage and on chip: 512x512x41 6.34 and 7.01 ms (19 units of
+// pencil_cost a level), 512x256x41 3.51 and 3.51 (21; option 2 is 5 % cheaper on
+// chip), 256x256x41 2.16 and 1.79; 128x128x16 with eight sources 1.34 and 1.79,
+// with one 0.44 and 0.26.  The line depends on the grid alone, so that a source's
+// arithmetic does not depend on the batch around it, and lies where neither one
+// source nor eight lose on chip: up to 20 levels from 4000 modes, and on the
+// largest grids the boxes that leave too many lanes empty (512x512: 25 to 28, 41
+// to 46, 81 to 92 levels and the like).
+bool stages_faster(int option, int modes, int nz, const PencilShape& sh) {
+    if (modes >= 46000) return (option == 2 ? 0.95 : 1.0) * pencil_cost(sh) > (modes >= 92000 ? 19.0 : 21.2) * nz;
+    return modes >= 4000 && nz <= 20;
 }
 
 // The scheme's solves for y = f' - (C2/alpha) d1, d1(j) = f(j+1) - f(j-1):
@@ -265,14 +281,14 @@ std::vector<double> z_table(int nz, const std::vector<double>& stretch, const Tr
 
 // Values of the table of pencil.cu
 size_t pencil_table_size(const PencilShape& sh, int nzpml) {
-    const size_t tp = 32 * sh.W;
+    const size_t tp = sh.tp;
     return PZ_COUNT * tp * sh.ch + 2 * PC_COUNT * tp + 4 * PE_COUNT + 3 * (size_t)nzpml;
 }
 
 // The table of pencil.cu (its order: internal.cuh)
 std::vector<double> pencil_table(int nz, int nb, int nt, const PencilShape& sh, int option, const double* zt,
                                  const Tri* tri, const Compact<double>& cc) {
-    const int ch = sh.ch, tp = 32 * sh.W, nzp = tp * ch, nzpml = nb + nt;
+    const int ch = sh.ch, tp = sh.tp, seg = std::min(tp, 32), nzp = tp * ch, nzpml = nb + nt;
     std::vector<double> tab(pencil_table_size(sh, nzpml), 0.0);
     auto put = [&](int row, int j, double v) { tab[(size_t)row * nzp + (size_t)(j % ch) * tp + j / ch] = v; };
     auto Z = [&](int row, int j) { return zt[(size_t)row * nz + j]; };
@@ -311,18 +327,18 @@ std::vector<double> pencil_table(int nz, int nb, int nt, const PencilShape& sh, 
         auto Mc = [&](int t) { return r.HH[(size_t)t * ch + ch - 1]; };
         auto Gc = [&](int t) { return r.GG[(size_t)t * ch]; };
         for (int t = 0; t < tp; ++t) {
-            const int lane = t % 32, w0 = t - lane;
+            const int lane = t % seg, w0 = t - lane;      // lane among the pencil's lanes of the warp
             for (int q = 0; q < 4; ++q) {
                 const int d = 1 << q;
-                double f = lane >= d ? 1.0 : 0.0, b = lane + d <= 31 ? 1.0 : 0.0;
+                double f = lane >= d ? 1.0 : 0.0, b = lane + d < seg ? 1.0 : 0.0;
                 for (int i = 1; i <= d && lane >= d; ++i) f *= Mc(t - i);
-                for (int i = 1; i <= d && lane + d <= 31; ++i) b *= Gc(t + i);
+                for (int i = 1; i <= d && lane + d < seg; ++i) b *= Gc(t + i);
                 c[(size_t)(PC_F + q) * tp + t] = f;
                 c[(size_t)(PC_B + q) * tp + t] = b;
             }
             double fw = 1.0, bw = 1.0;
             for (int i = w0; i < t; ++i) fw *= Mc(i);
-            for (int i = t + 1; i < w0 + 32; ++i) bw *= Gc(i);
+            for (int i = t + 1; i < w0 + seg; ++i) bw *= Gc(i);
             c[(size_t)PC_FL * tp + t] = Mc(t);
             c[(size_t)PC_FW * tp + t] = fw;
             c[(size_t)PC_BL * tp + t] = Gc(t);
@@ -547,10 +563,11 @@ int sparc_gpu_create(const sparc_params* p, sparc_ctx** out) {
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, dev);
         cudaGetLastError();
         const int opt = p->option, bc1 = opt == 17 ? 3 : 1, bc2 = opt == 17 ? 2 : 0;
-        c->pencil = pencil_shape(c->nz, c->M);
+        c->pencil = pencil_shape(c->nz, c->M, !c->f32, c->nsm);
         c->use_pencil = (opt == 2 || (!c->f32 && (opt == 4 || opt == 17))) &&
                         getenv(c->f32 ? "SPARC_FP32_PER_STAGE" : "SPARC_STAGE_LANES") == nullptr &&
                         pencil_count(c->pencil, opt, c->nzpml, (int)cs, 1, c->nsm) > 0 &&
+                        (c->f32 || !stages_faster(opt, c->M, c->nz, c->pencil)) &&
                         pencil_ok(c->nz, c->pencil, bc1, bc2) &&
                         (c->f32 ? pencil_prepare<float>(c->pencil, opt)
                                 : pencil_prepare<double>(c->pencil, opt));
@@ -1253,7 +1270,8 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
         B.tab = (const T*)c->ptab; B.pt = A.pt;
         B.fs = A.fs; B.ps = A.ps; B.M = A.M; B.nz = A.nz; B.nzpml = c->nzpml;
         B.npmlbot = A.npmlbot; B.npmltop = A.npmltop; B.option = A.option; B.damp = A.damp;
-        B.W = c->pencil.W;
+        B.W = std::max(1, c->pencil.tp / 32);
+        B.part = c->pencil.tp < 32 ? c->pencil.tp : 0;
         B.nsrc = c->active_n;
         B.pencils = c->pencil_tuned ? c->pencil_tuned
                                     : pencil_count(c->pencil, A.option, c->nzpml, (int)csz(c),
@@ -1415,7 +1433,7 @@ static void set_variant(sparc_ctx* c, int v) {
     }
     c->stage_block = v;
     if (c->use_pencil)
-        c->pencil_tuned = std::min(std::max(1, v / (32 * c->pencil.W)),
+        c->pencil_tuned = std::min(std::max(pencil_least(c->pencil), v / c->pencil.tp),
                                    pencil_count(c->pencil, c->P.option, c->nzpml, (int)csz(c), 1LL << 40, c->nsm));
 }
 

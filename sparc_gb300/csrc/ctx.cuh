@@ -42,7 +42,7 @@ struct sparc_ctx {
     int use_fused = 0;
     int fused_pencils = 4;                        // modes per CTA of the fused step (autotuned)
     int use_pencil = 0;                           // whole-step kernel of pencil.cu
-    PencilShape pencil = {5, 1};
+    PencilShape pencil = {5, 32};
     int pencil_tuned = 0;                         // pencils per CTA picked by the autotuner (0: by rule)
     void* ptab = nullptr;                         // its T table
     int nsm = 152;                                // SMs of the device

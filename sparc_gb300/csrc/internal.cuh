@@ -412,7 +412,7 @@ enum {      // carry rows: products of chunk multipliers
 // closure coefficients of one end: the second row from the end (five), the
 // end row (five), and the factor of a caller-set end value
 enum { PE_TOP = 10, PE_COUNT = 12 };
-struct PencilShape { int ch, W; };      // levels per thread, warps per pencil
+struct PencilShape { int ch, tp; };     // levels per thread, threads per pencil (8, 16, or whole warps)
 template <typename T> struct PencilArgs {
     typedef typename CplxOf<T>::type CT;
     CT* a; CT* scr; CT* pml;
@@ -430,8 +430,11 @@ template <typename T> struct PencilArgs {
     CT* rec;            // surface records, as FusedArgs
     int rec_steps, rec_max, rec_k;
     SlotClock clk;
+    int part;           // lanes of a pencil that takes a part of a warp (W = 1), else 0
 };
-PencilShape pencil_shape(int nz, int modes);
+PencilShape pencil_shape(int nz, int modes, bool f64, int nsm);
+double pencil_cost(const PencilShape& sh);
+inline int pencil_least(const PencilShape& sh) { return sh.tp < 32 ? 32 / sh.tp : 1; }   // pencils of a warp: the fewest a CTA takes
 int pencil_count(const PencilShape& sh, int option, int nzpml, int complex_bytes, long long pencils, int nsm);
 template <typename T> int pencil_prepare(const PencilShape& sh, int option);
 template <typename T> void launch_pencil(const PencilArgs<T>& A, int ch, cudaStream_t s);

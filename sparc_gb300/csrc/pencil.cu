@@ -3,7 +3,8 @@
 // and 17 have fused.cu.
 //
 // Layout.  A pencil (one horizontal mode of one source) is cut into chunks of
-// CH levels, one per thread: TP = 32 W threads, padded to TP CH levels.  `a`
+// CH levels, one per thread: TP threads (whole warps, or in FP64 a
+// half or a quarter of one: two or four pencils a warp), padded to TP CH levels.  `a`
 // sits in shared memory as [field][pencil][chunk], scr in registers, the PML
 // planes in shared memory; a CTA holds P pencils.  A pencil's step needs
 // nothing of another pencil, so a launch takes up to FUSED_STEPS steps before
@@ -37,11 +38,12 @@
 // rounding of FP64; the host checks that bound for the boundary codes in use
 // (else the per-stage kernels run).
 //
-// Chunk length (pencil_shape): 3 to 7 levels, whichever leaves the fewest
-// lanes without levels; it depends on the grid only, so a source's arithmetic
-// does not depend on the batch around it.  Chunks are stored CHP = CH or CH+1
-// (odd) values apart, which keeps the 16-byte accesses of a warp free of bank
-// conflicts.
+// Shape (pencil_shape): the levels per thread and threads per pencil of the least
+// issue cost, on grids with few modes those of the shortest chain; it depends on
+// the grid only, so a source's arithmetic does not depend on the batch around it.
+// Chunks are stored CHP = CH or CH+1 (odd) values apart, which keeps the 16-byte
+// accesses of a warp free of bank conflicts.  Where the per-stage kernels are
+// faster (few levels and many modes), capi.cu keeps to them.
 //
 // Measured per step, against one launch per stage with the pencils in HBM:
 // 128x128x150, one source, FP64 2.40 -> 1.36 ms; 256x256x300 FP64 adjoint
@@ -70,31 +72,31 @@ __device__ __forceinline__ CT ifma(T k, CT v, CT a) {
     return r;
 }
 
-template <typename CT> __device__ __forceinline__ CT shfl_up_c(CT v, int d) {
+// the value d lanes below / above, of the same pencil (seg lanes of the warp hold one)
+template <typename CT> __device__ __forceinline__ CT shfl_up_c(CT v, int d, int seg) {
     CT r;
-    r.x = __shfl_up_sync(0xffffffffu, v.x, d);
-    r.y = __shfl_up_sync(0xffffffffu, v.y, d);
+    r.x = __shfl_up_sync(0xffffffffu, v.x, d, seg);
+    r.y = __shfl_up_sync(0xffffffffu, v.y, d, seg);
     return r;
 }
-template <typename CT> __device__ __forceinline__ CT shfl_down_c(CT v, int d) {
+template <typename CT> __device__ __forceinline__ CT shfl_down_c(CT v, int d, int seg) {
     CT r;
-    r.x = __shfl_down_sync(0xffffffffu, v.x, d);
-    r.y = __shfl_down_sync(0xffffffffu, v.y, d);
+    r.x = __shfl_down_sync(0xffffffffu, v.x, d, seg);
+    r.y = __shfl_down_sync(0xffffffffu, v.y, d, seg);
     return r;
 }
 
-// Barrier over the TP threads of one pencil (a named barrier; one warp needs none).
+// Barrier over the TP threads of one pencil (a named barrier; one warp or a part of one needs none).
 __device__ __forceinline__ void pencil_sync(int pi, int tp) {
-    if (tp == 32) __syncwarp();
+    if (tp <= 32) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(pi + 1), "r"(tp) : "memory");
 }
 
 struct PencilLayout {      // offsets in complex values, identical on host and device
     int tile, xf, xb, cl, pd, ptile, spt, cells, total, LZ, LX;
 };
-__host__ __device__ inline PencilLayout pencil_layout(int P, int W, int CH, int nzpml, int option) {
+__host__ __device__ inline PencilLayout pencil_layout(int P, int TP, int CH, int nzpml, int option) {
     PencilLayout L;
-    const int TP = 32 * W;
     L.LZ = (TP + 2 * GC) * (CH | 1);
     L.LX = TP + 2;
     int o = 0;
@@ -105,7 +107,7 @@ __host__ __device__ inline PencilLayout pencil_layout(int P, int W, int CH, int 
     L.pd = o;    o += P * nzpml;         // exchange of the PML planes
     L.ptile = o; o += 2 * nzpml * P;     // [pencil][2][plane]
     L.spt = o;   o += 2 * nzpml * P;
-    L.cells = o; o += 2 * P * W;         // forward and backward carries between warps
+    L.cells = o; o += 2 * P * ((TP + 31) / 32);         // forward and backward carries between warps
     L.total = o;
     return L;
 }
@@ -116,14 +118,14 @@ __host__ __device__ inline PencilLayout pencil_layout(int P, int W, int CH, int 
 // j0..j0+CH-1.  top: the caller-set value of bc 3.  zt: the thread's column
 // of the elimination rows (row stride NZP, level q at q TP), ct: of the carry
 // rows (row stride TP), ce: the closure coefficients of this solve.
-template <int CH, typename T, typename CT>
+template <int CH, bool PART, typename T, typename CT>
 __device__ __forceinline__ void pencil_solve(const CT (&own)[CH], CT left, CT right, const CT* cl,
                                              const T* __restrict__ zt, const T* __restrict__ ct,
                                              const T* __restrict__ ce, bool has_top, CT top, int NZP, int TP, int nz,
                                              int j0, bool lo, bool hi, int t, CT* cf, CT* cb, int pi, CT (&out)[CH]) {
     auto Z = [&](int row, int q) -> T { return __ldg(&zt[row * NZP + q * TP]); };
     auto C = [&](int row) -> T { return __ldg(&ct[row * TP]); };
-    const int lane = t & 31, w = t >> 5;
+    const int lane = t & 31, w = t >> 5, seg = PART ? TP : 32;
     CT d1[CH], u[CH];
     #pragma unroll
     for (int q = 0; q < CH; ++q) {
@@ -156,10 +158,10 @@ __device__ __forceinline__ void pencil_solve(const CT (&own)[CH], CT left, CT ri
     }
     // carry from the chunks below: exclusive scan over 16 chunks of the warp,
     // then the last value of the warp below
-    CT e = shfl_up_c(run, 1);
+    CT e = shfl_up_c(run, 1, seg);
     if (lane == 0) e = czero<CT>();
     #pragma unroll
-    for (int k = 0; k < 4; ++k) e = cfma(C(PC_F + k), shfl_up_c(e, 1 << k), e);   // zero coefficient where it leaves the warp
+    for (int k = 0; k < 4; ++k) e = cfma(C(PC_F + k), shfl_up_c(e, 1 << k, seg), e);   // zero coefficient where it leaves the pencil's lanes
     if (TP > 32 && lane == 31) cf[w] = cfma(C(PC_FL), e, run);
     // back substitution with zero carries
     CT x = u[CH - 1];
@@ -173,10 +175,10 @@ __device__ __forceinline__ void pencil_solve(const CT (&own)[CH], CT left, CT ri
     if (w > 0) e = cfma(C(PC_FW), cf[w - 1], e);
     // y(j) = x0(j) + K(j) e + G(j) f, f the carry from the chunks above
     x = cfma(Z(PS_K, 0), e, x);
-    CT f = shfl_down_c(x, 1);
-    if (lane == 31) f = czero<CT>();
+    CT f = shfl_down_c(x, 1, seg);
+    if (lane == seg - 1) f = czero<CT>();
     #pragma unroll
-    for (int k = 0; k < 4; ++k) f = cfma(C(PC_B + k), shfl_down_c(f, 1 << k), f);
+    for (int k = 0; k < 4; ++k) f = cfma(C(PC_B + k), shfl_down_c(f, 1 << k, seg), f);
     if (TP > 32) {
         if (lane == 0) cb[w] = cfma(C(PC_BL), f, x);
         pencil_sync(pi, TP);
@@ -193,7 +195,8 @@ __device__ __forceinline__ void pencil_solve(const CT (&own)[CH], CT left, CT ri
 // (xi_y), xi_z, v_x, (v_y), v_z; 2: rho, v_x, v_y, v_z, p, (unused), then v
 // along k.  The fields in brackets have no right-hand side: they are only
 // filtered, and only where a CTA holds a non-zero value of them.
-template <typename T, int FORM, int CH>
+// PART: a pencil takes a part of a warp (seg lanes of it).
+template <typename T, int FORM, int CH, bool PART>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kernel(const PencilArgs<T> A) {
     typedef typename CplxOf<T>::type CT;
     constexpr bool D3 = FORM != 17, VEL = FORM == 2;
@@ -203,10 +206,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
     constexpr int FZ = VEL ? 2 : 1;                       // sc index of the field the first solve differentiates
     constexpr int FV = VEL ? 2 : 3;                       // sc index of v_z
     extern __shared__ __align__(16) unsigned char smraw[];
-    const int W = A.W, P = A.pencils, TP = 32 * W, NZP = TP * CH;
+    const int W = A.W, P = A.pencils, TP = PART ? A.part : 32 * W, NZP = TP * CH;
     const int nz = A.nz, M = A.M, nzpml = A.nzpml, nb = A.npmlbot, nt = A.npmltop;
     const long long fs = A.fs;
-    const PencilLayout Ly = pencil_layout(P, W, CH, nzpml, FORM);
+    const PencilLayout Ly = pencil_layout(P, TP, CH, nzpml, FORM);
     const int LZ = Ly.LZ, FT = P * LZ;                    // field stride of the tile
     CT* sm = (CT*)smraw;
     CT* tile = sm + Ly.tile;
@@ -270,7 +273,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
 
     const bool lo = j0 == 0, hi = j0 <= nz - 1 && j0 + CH > nz - 2;
     // PML levels of this chunk: bit q of pmask, plane index pipv + q; and the
-    // planes of this warp's levels: nbw bottom ones from plane pb, ntw top ones from plane pt
+    // planes of the levels of this pencil's lanes in the warp: nbw bottom ones from plane pb, ntw top ones from plane pt
     unsigned pmask = 0;
     int pipv = 0;
     if (j0 < nb) {
@@ -283,7 +286,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
             pipv = nb + (j0 - (nz - nt));
         }
     }
-    const int lane = t & 31, wl = (t - lane) * CH, wh = wl + 32 * CH;
+    const int lane = t & 31, seg = PART ? TP : 32, wl = (t - lane) * CH, wh = wl + seg * CH;
     const int nbw = max(0, min(nb, wh) - wl), tl_ = max(nz - nt, wl), ntw = max(0, min(nz, wh) - tl_);
     const int npw = nbw + ntw;
     auto plane = [&](int i) { return i < nbw ? wl + i : nb + tl_ - (nz - nt) + (i - nbw); };
@@ -341,7 +344,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
         // psi of the PML planes of auxiliary k (psi_vz, psi_p): right-hand side a d + b psi, psi back in pd
         auto pml = [&](int k, const T* az) {
             __syncwarp();
-            for (int i = lane; i < npw; i += 32) {
+            for (int i = lane; i < npw; i += seg) {
                 const int ip = plane(i), o = k * nzpml + ip;
                 CT psi = ptile[o];
                 if (hs) psi = cfma(beta, spt[o], psi);
@@ -360,7 +363,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
                 if (j0 + q == nz - 1) top = cscale(-A.unstr_top, ifma(kap, arg(F0, 0, q), czero<CT>()));
         }
         exchange(own);
-        pencil_solve<CH, T, CT>(own, xb[t - 1], xf[t + 1], cl, zt + PZ_S1 * NZP, c1, ce, FORM == 17, top, NZP, TP, nz,
+        pencil_solve<CH, PART, T, CT>(own, xb[t - 1], xf[t + 1], cl, zt + PZ_S1 * NZP, c1, ce, FORM == 17, top, NZP, TP, nz,
                                 j0, lo, hi, t, cf, cb, pi, d);
         if (npw) {                   // psi_vz
             #pragma unroll
@@ -400,7 +403,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
         }
         exchange(own);
         // d: stretch / rho0 times d/dz of p'
-        pencil_solve<CH, T, CT>(own, xb[t - 1], xf[t + 1], cl, zt + PZ_S2 * NZP, c2, ce + 2 * PE_COUNT, false,
+        pencil_solve<CH, PART, T, CT>(own, xb[t - 1], xf[t + 1], cl, zt + PZ_S2 * NZP, c2, ce + 2 * PE_COUNT, false,
                                 czero<CT>(), NZP, TP, nz, j0, lo, hi, t, cf, cb, pi, d);
         #pragma unroll
         for (int q = 0; q < CH; ++q)
@@ -524,7 +527,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
             }
         }
         // pml += dt*scrpml (step.f90:116)
-        for (int i = lane; i < 2 * npw; i += 32) {
+        for (int i = lane; i < 2 * npw; i += seg) {
             const int o = (i < npw ? 0 : nzpml) + plane(i < npw ? i : i - npw);
             ptile[o] = cfma(A.dt, spt[o], ptile[o]);
         }
@@ -595,72 +598,108 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) pencil_step_kerne
     }
 }
 
-// FP32 is built for the velocity form alone
-template <typename T, int CH>
-const void* kernel_ch(int option) {
+// FP32 is built for the velocity form alone, parts of a warp for FP64 with up to
+// five levels a thread (pencil_shape)
+template <typename T, int CH, bool PART>
+const void* kernel_form(int option) {
     if constexpr (sizeof(T) == 8) {
-        if (option == 17) return (const void*)pencil_step_kernel<T, 17, CH>;
-        if (option == 4) return (const void*)pencil_step_kernel<T, 4, CH>;
+        if (option == 17) return (const void*)pencil_step_kernel<T, 17, CH, PART>;
+        if (option == 4) return (const void*)pencil_step_kernel<T, 4, CH, PART>;
     }
-    return (const void*)pencil_step_kernel<T, 2, CH>;
+    return (const void*)pencil_step_kernel<T, 2, CH, PART>;
+}
+template <typename T, int CH>
+const void* kernel_ch(int option, int tp) {
+    if constexpr (sizeof(T) == 8 && CH <= 5) {
+        if (tp < 32) return kernel_form<T, CH, true>(option);
+    }
+    return kernel_form<T, CH, false>(option);
 }
 template <typename T>
-const void* kernel_of(int option, int ch) {
-    switch (ch) {
-        case 3: return kernel_ch<T, 3>(option);
-        case 4: return kernel_ch<T, 4>(option);
-        case 6: return kernel_ch<T, 6>(option);
-        case 7: return kernel_ch<T, 7>(option);
-        default: return kernel_ch<T, 5>(option);
+const void* kernel_of(int option, const PencilShape& sh) {
+    switch (sh.ch) {
+        case 3: return kernel_ch<T, 3>(option, sh.tp);
+        case 4: return kernel_ch<T, 4>(option, sh.tp);
+        case 6: return kernel_ch<T, 6>(option, sh.tp);
+        case 7: return kernel_ch<T, 7>(option, sh.tp);
+        default: return kernel_ch<T, 5>(option, sh.tp);
     }
 }
 
 size_t pencil_bytes(const PencilShape& sh, int option, int P, int nzpml, int complex_bytes) {
-    return (size_t)pencil_layout(P, sh.W, sh.ch, nzpml, option).total * complex_bytes;
+    return (size_t)pencil_layout(P, sh.tp, sh.ch, nzpml, option).total * complex_bytes;
 }
 
 }  // namespace
 
-// Levels per thread and warps per pencil of a grid: the least cost of a
-// pencil's step, counted as warps times the FP64 instructions of a thread
-// (per chunk 40 a stage for the scans and 60 for closures and PML, per level
-// 55 a stage and 144 for update and filter).  On grids with few modes (an SM
-// holds no more than four pencils of one source) a step is the length of its
-// serial chains: 3 levels per thread, as many warps as that takes.
-PencilShape pencil_shape(int nz, int modes) {
-    PencilShape best = {5, (nz + 159) / 160};
+// Cost of a pencil's step of a shape: warps times the FP64 instructions of a thread
+// (per chunk 40 a stage for the scans and 60 for closures and PML, per level 55 a
+// stage and 144 for update and filter).  A step takes 4.05 us a unit to within 4 %
+// on every shape of option 4 at 512x256.
+double pencil_cost(const PencilShape& sh) { return sh.tp / 32.0 * (5 * 100.0 + sh.ch * (5 * 55.0 + 144.0)); }
+
+// Levels per thread and threads per pencil of a grid: the least cost.  FP64
+// issue pays for a lane without levels as for a full one, so boxes of up to 40
+// levels take a quarter and of up to 80 half of a warp (512x256, option 4, ms a step
+// with a whole warp and so: 24 levels 6.94 and 1.84, 48 levels 6.94 and 3.51, 80
+// levels 6.94 and 5.21); with 6 or 7 levels a thread such pencils leave an SM four
+// or five warps, too few (96 levels on half a warp 7.02, on a whole one 6.94).
+// FP32 (option 2) is not bound by FP64 and keeps whole warps.  On grids with few
+// modes (an SM holds no more than four pencils of one source) a step is the length
+// of its serial chains: 3 levels per thread, as many lanes as that takes
+// (256x1x300, one source: 3 levels on four warps 69 us, 4 on three 80, 5 on two
+// 93; eight sources, which fill the GPU, 376, 389 and 329: the shape depends on
+// the grid alone, so that a source's arithmetic does not depend on the batch
+// around it).
+PencilShape pencil_shape(int nz, int modes, bool f64, int nsm) {
+    PencilShape best = {5, 32 * ((nz + 159) / 160)};
     double cost = 0.0;
+    const bool few = modes <= 4 * nsm;
     for (int ch = 3; ch <= 7; ++ch) {
-        const int W = (nz + 32 * ch - 1) / (32 * ch);
-        if (W > 8 || (modes <= 608 && ch > 3 && (nz + 95) / 96 <= 8)) continue;
-        const double c = W * (5 * 100.0 + ch * (5 * 55.0 + 144.0));
-        if (cost == 0.0 || c < cost) { cost = c; best = {ch, W}; }
+        const bool part = f64 && ch <= 5 && nz <= 16 * ch;
+        const PencilShape sh = {ch, part ? (nz <= 8 * ch ? 8 : 16) : 32 * ((nz + 32 * ch - 1) / (32 * ch))};
+        if (sh.tp > 256 || (few && ch > 3 && (nz + 95) / 96 <= 8)) continue;
+        const double c = pencil_cost(sh);
+        if (cost == 0.0 || c < cost) { cost = c; best = sh; }
     }
     return best;
 }
 
 // Pencils per CTA: 128 threads (two CTAs an SM overlap one's copies with the
-// other's arithmetic), fewer when the launch would leave SMs without two CTAs.
-// 0: not even one pencil fits the shared memory a CTA may use.
+// other's arithmetic), fewer when the launch would leave SMs without two CTAs;
+// whole warps.  Part-warp pencils take the size of which an SM holds most warps
+// (8 at the kernel's 255 registers), the larger of two that give as many, and two
+// warps a CTA at least: CTAs of one warp are a sixth slower (512x256x48, half a
+// warp a pencil: 8 or 4 pencils a CTA 3.51 ms a step, 2 pencils 4.13).
+// 0: not even one warp fits the shared memory a CTA may use.
 int pencil_count(const PencilShape& sh, int option, int nzpml, int complex_bytes, long long pencils, int nsm) {
-    if (32 * sh.W > 256 || pencil_bytes(sh, option, 1, nzpml, complex_bytes) > 227 * 1024) return 0;
-    int P = std::max(1, 128 / (32 * sh.W));
-    while (P > 1 && (pencil_bytes(sh, option, P, nzpml, complex_bytes) > 113 * 1024 || (pencils + P - 1) / P < 2LL * nsm))
-        P /= 2;
+    const int least = pencil_least(sh);
+    auto bytes = [&](int p) { return pencil_bytes(sh, option, p, nzpml, complex_bytes); };
+    if (sh.tp > 256 || bytes(least) > 227 * 1024) return 0;
+    int P = std::max(least, 128 / sh.tp);
+    if (sh.tp < 32) {
+        int held = 0;
+        for (int p = 128 / sh.tp; p >= 2 * least; p /= 2) {
+            const int warps = std::min(8, (int)(228 * 1024 / (bytes(p) + 1024)) * (p / least));
+            if (warps > held) { held = warps; P = p; }
+        }
+    }
+    while (P > least && (bytes(P) > 113 * 1024 || (pencils + P - 1) / P < 2LL * nsm)) P /= 2;
     return P;
 }
 
 template <typename T>
 int pencil_prepare(const PencilShape& sh, int option) {
-    return allow_shared_memory(kernel_of<T>(option, sh.ch));
+    return allow_shared_memory(kernel_of<T>(option, sh));
 }
 
 template <typename T>
 void launch_pencil(const PencilArgs<T>& A, int ch, cudaStream_t s) {
-    const size_t smem = pencil_bytes({ch, A.W}, A.option, A.pencils, A.nzpml, 2 * sizeof(T));
+    const PencilShape sh = {ch, A.part ? A.part : 32 * A.W};
+    const size_t smem = pencil_bytes(sh, A.option, A.pencils, A.nzpml, 2 * sizeof(T));
     const long long ctas = (long long)((A.M + A.pencils - 1) / A.pencils) * A.nsrc;
     void* args[] = {(void*)&A};
-    cudaLaunchKernel(kernel_of<T>(A.option, ch), dim3((unsigned)ctas), dim3(A.pencils * 32 * A.W), args, smem, s);
+    cudaLaunchKernel(kernel_of<T>(A.option, sh), dim3((unsigned)ctas), dim3(A.pencils * sh.tp), args, smem, s);
 }
 
 template int pencil_prepare<double>(const PencilShape&, int);
