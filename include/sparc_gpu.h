@@ -153,9 +153,10 @@ int sparc_gpu_set_mhd2d_background(sparc_ctx* ctx, const double* rho, const doub
                                    const double* psi);
 
 /* Pick the fastest of the launch variants that give identical results (the
- * fused FP32 step's modes per CTA, 4 or 2; the per-stage kernels' threads per
- * CTA, 128 or 64) by timing real steps: the call advances the solution by
- * 4*steps ordinary time steps.  Steps are replayed from captured CUDA graphs
+ * fused FP32 step's modes per CTA, 4, 2 or 8; the other kernels' threads per
+ * CTA, 128, 64 or 32, in pencil.cu the whole pencils that fill them) by timing
+ * real steps: the call advances the solution by 2*steps ordinary time steps per
+ * variant.  Steps are replayed from captured CUDA graphs
  * (one per step count, captured on first use and after any change of launch
  * arguments); SPARC_NO_GRAPHS in the environment at create time launches
  * them directly.  choice / ms_per_step may be NULL.  No reference

@@ -1425,16 +1425,15 @@ int sparc_gpu_set_mhd_background(sparc_ctx* c, const double* rho, const double* 
 }
 
 // A launch variant of the autotuner: modes per CTA of the fused step, threads
-// per CTA of the other step kernels (the pencils that fill them in pencil.cu)
-static void set_variant(sparc_ctx* c, int v) {
-    if (c->use_fused && c->f32) {
-        c->fused_pencils = v;
-        return;
-    }
+// per CTA of the other step kernels.  pencil.cu takes the whole pencils that fill
+// them, one at least; returns what is then launched
+static int set_variant(sparc_ctx* c, int v) {
+    if (c->use_fused && c->f32) return c->fused_pencils = v;
     c->stage_block = v;
-    if (c->use_pencil)
-        c->pencil_tuned = std::min(std::max(pencil_least(c->pencil), v / c->pencil.tp),
-                                   pencil_count(c->pencil, c->P.option, c->nzpml, (int)csz(c), 1LL << 40, c->nsm));
+    if (!c->use_pencil) return v;
+    c->pencil_tuned = std::min(std::max(pencil_least(c->pencil), v / c->pencil.tp),
+                               pencil_count(c->pencil, c->P.option, c->nzpml, (int)csz(c), 1LL << 40, c->nsm));
+    return c->pencil_tuned * c->pencil.tp;
 }
 
 int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step) {
@@ -1467,11 +1466,11 @@ int sparc_gpu_autotune(sparc_ctx* c, int steps, int* choice, float* ms_per_step)
         ms /= steps;
         if (v == cand[0] || ms < best) { best = ms; pick = v; }
     }
-    set_variant(c, pick);
+    const int ran = set_variant(c, pick);
     c->epoch++;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (choice) *choice = pick;
+    if (choice) *choice = ran;
     if (ms_per_step) *ms_per_step = best;
     return SPARC_OK;
 }

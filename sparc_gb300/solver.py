@@ -119,12 +119,12 @@ class Solver:
 
     def autotune(self, steps: int = 1) -> dict:
         """Time each launch variant that gives identical results over real
-        steps (4*steps of them) and keep the fastest; returns the choice."""
+        steps (2*steps of them for each) and keep the fastest; returns the choice."""
         choice = ctypes.c_int(0)
         ms = ctypes.c_float(0.0)
         self._ck(self.L.sparc_gpu_autotune(self.h, int(steps), ctypes.byref(choice), ctypes.byref(ms)))
-        fused = self.p.nz <= (480 if self.p.option == 4 else 320)
-        key = "modes_per_cta" if (self.p.precision == "f32" and fused) else "threads_per_cta"
+        fused = self.p.precision == "f32" and self.p.nz <= {4: 480, 17: 320}.get(self.p.option, 0)
+        key = "modes_per_cta" if fused else "threads_per_cta"
         return {key: choice.value, "ms_per_step": ms.value}
 
     def stage(self, rk: int):
