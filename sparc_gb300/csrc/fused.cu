@@ -52,8 +52,8 @@
 //     tables solve for the scaled unknown s(j) x(j) (s = stretch for xi_z,
 //     stretch / rho0 for p'), so each solve returns the derivative in the
 //     form the step uses, without a multiply and a table read per level;
-//   * the state tile of the CTA that starts one resident-CTA count later is
-//     prefetched into L2 while this CTA computes, so its load phase reads L2;
+//   * in a launch of one step the state tile of a CTA's next item is prefetched
+//     into L2 while this one is computed, so its load phase reads L2;
 //   * a LAGRANGE_INTERP source (the adjoint's) is interpolated to the step by
 //     a small kernel launched before it (source_plane_kernel), so no CTA
 //     spends its critical path on the seven FP64 weights.
@@ -62,8 +62,8 @@
 //     storing the tile, and the z tables, took a quarter of a CTA's time when
 //     every step did it.  Measured per step: 256x256x300, 8 sources 5.55 ->
 //     4.19 ms; 512x512x300, one adjoint source 2.99 -> 2.10 ms; results bit
-//     for bit the same.  The limit bounds a CTA's time (about half a
-//     millisecond), after which launches of other streams get its SM.
+//     for bit the same.  The limit bounds a CTA's time (0.3 ms at
+//     256x256x300), after which launches of other streams get its SM.
 // HBM traffic per launch: read a, write a (+ the PML planes and source planes),
 // and scr only on steps whose right-hand side is requested (outputs).
 #include <algorithm>
@@ -386,8 +386,8 @@ __global__ void __launch_bounds__(P * 32 * W, fused_ctas(P, W, CH)) fused_step_k
             return;
         }
 
-        // ---- L2 prefetch of the rows of the CTA that starts pf_stride CTAs
-        // later (about when this one ends): its tile load then comes from L2 ----
+        // ---- L2 prefetch of the rows of this CTA's next item (launches of one step;
+        // a launch of several has none): its tile load then comes from L2 ----
         if (A.pf_stride > 0) {
             const int nid = item + gridDim.x;             // this CTA's next item
             if (nid < nitem) {

@@ -368,10 +368,16 @@ struct FusedArgs {
     float2* rec;        // surface records [S][rec_max][M], or null: v_z at level rec_k every rec_steps steps
     int rec_steps, rec_max, rec_k;
     int nsrc;           // sources of the launch (set by the launcher)
-    int pf_stride;      // > 0: each CTA prefetches into L2 the rows of the CTA pf_stride later in launch
-                        // order (set by the launcher to the CTAs resident at once); 0: no prefetch
+    int pf_stride;      // > 0: each CTA prefetches into L2 the rows of its next item; 0: no prefetch
 };
 constexpr int FUSED_STEPS = 16;   // time steps of one launch of the whole-step kernels, at most
+// and of pencil.cu in FP64 where a launch fills the GPU twice (8 warps an SM).  A CTA
+// keeps its place until its steps are done, and an FP64 step is long: 15 steps of a
+// more urgent FP32 context of 64x64x75 take 0.5 ms alone and, beside FP64 contexts of
+// 128x128x150 or 256x256x300, 5.4 ms with 16 steps a launch, 2.6 with 8 and 1.3 with
+// 4 (2.2 and 1.2 beside one launch per stage); a step of the FP64 context costs
+// 0.4 % more with 8 and 1 % with 4
+constexpr int PENCIL_STEPS = 4;
 struct FusedShape { int ch, W; }; // levels per thread, warps per pencil
 FusedShape fused_shape(int nz, bool d3);   // d3: option 4, else 17
 int fused_nzp(int nz, bool d3);            // padded levels
