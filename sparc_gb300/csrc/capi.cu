@@ -1287,9 +1287,9 @@ static int enqueue_steps(sparc_ctx* c, int nsteps) {
             B.rec = CP<T>(c->rec); B.rec_steps = c->steps; B.rec_max = c->rec_max; B.rec_k = c->o_rad - 1;
         }
         B.clk = A.clk;
-        const bool fills = !c->f32 && (long long)c->M * c->active_n * c->pencil.tp >= 32LL * 16 * c->nsm;
+        const int most = c->f32 ? FUSED_STEPS : pencil_steps((long long)c->M * c->active_n * c->pencil.tp / 32 / c->nsm);
         for (int it = 0; it < nsteps; it += B.nsteps) {
-            B.nsteps = std::min(nsteps - it, fills ? PENCIL_STEPS : FUSED_STEPS);
+            B.nsteps = std::min(nsteps - it, most);
             B.write_scr = (it + B.nsteps == nsteps && c->rhs_out) ? 1 : 0;
             if (B.src_mode == 2) {
                 launch_source_plane<T>(B.src_plane, B.planes, B.plane_ss, B.L, B.clk, c->M, B.nsteps, c->active_n,

@@ -371,13 +371,14 @@ struct FusedArgs {
     int pf_stride;      // > 0: each CTA prefetches into L2 the rows of its next item; 0: no prefetch
 };
 constexpr int FUSED_STEPS = 16;   // time steps of one launch of the whole-step kernels, at most
-// and of pencil.cu in FP64 where a launch fills the GPU twice (8 warps an SM).  A CTA
+// and of pencil.cu in FP64, by the warps of a launch per SM (8 fit at a time).  A CTA
 // keeps its place until its steps are done, and an FP64 step is long: 15 steps of a
 // more urgent FP32 context of 64x64x75 take 0.5 ms alone and, beside FP64 contexts of
 // 128x128x150 or 256x256x300, 5.4 ms with 16 steps a launch, 2.6 with 8 and 1.3 with
-// 4 (2.2 and 1.2 beside one launch per stage); a step of the FP64 context costs
-// 0.4 % more with 8 and 1 % with 4
-constexpr int PENCIL_STEPS = 4;
+// 4 (2.2 and 1.2 beside one launch per stage).  4 cost such a step 1 % more than 16,
+// but up to 5 % on launches of a few waves (32x32x200, four sources: 0.762 and 0.798
+// ms), which take 8
+inline int pencil_steps(long long warps_per_sm) { return warps_per_sm >= 48 ? 4 : warps_per_sm >= 16 ? 8 : FUSED_STEPS; }
 struct FusedShape { int ch, W; }; // levels per thread, warps per pencil
 FusedShape fused_shape(int nz, bool d3);   // d3: option 4, else 17
 int fused_nzp(int nz, bool d3);            // padded levels

@@ -8,7 +8,7 @@
 // sits in shared memory as [field][pencil][chunk], scr in registers, the PML
 // planes in shared memory; a CTA holds P pencils.  A pencil's step needs
 // nothing of another pencil, so a launch takes up to FUSED_STEPS steps
-// (PENCIL_STEPS where it fills the GPU twice) before the state goes back to HBM.
+// (pencil_steps in FP64) before the state goes back to HBM.
 //
 // What bounds it: FP64 issue.  GB300 issues two FP64 lanes a clock and SM, so
 // the kernel is written for few FP64 instructions per level and stage (63 in

@@ -55,10 +55,11 @@ def test_short_boxes_match_the_oracle(gpu_lib, oracle_mod, option, nx, ny, nz):
 
 
 @pytest.mark.parametrize("option", [4, 2])
-@pytest.mark.parametrize("nz", [20, 41, 75, 101])
+@pytest.mark.parametrize("nz", [20, 41, 75, 101, 150])
 def test_short_boxes_do_not_depend_on_the_batch(gpu_lib, option, nz):
     """A slot of a batch of three, reset while the others run, equals the same
-    run alone, bit for bit, and n steps of a call n calls of one step."""
+    run alone, bit for bit, and n steps of a call n calls of one step (launches of
+    16, 8 or 4 steps, by the size of the batch)."""
     from cases import random_state
     from sparc_gb300.solver import Solver
     def run(nsrc, calls):
