@@ -211,12 +211,12 @@ bool pencil_ok(int nz, const PencilShape& sh, int bc1, int bc2) {
 // pencils, and without a price for lanes that hold no level.  Measured per step of
 // option 4, per stage and on chip: 512x512x41 6.34 and 7.01 ms (19 units of
 // pencil_cost a level), 512x256x41 3.51 and 3.51 (21; option 2 is 5 % cheaper on
-// chip from half a warp on), 256x256x41 2.16 and 1.79; 128x128x16 with eight sources 1.34 and 1.79,
-// with one 0.44 and 0.26.  The line depends on the grid alone, so that a source's
-// arithmetic does not depend on the batch around it, and lies where neither one
-// source nor eight lose on chip: up to 20 levels from 4000 modes, and on the
-// largest grids the boxes that leave too many lanes empty (512x512: 25 to 28, 41
-// to 46, 81 to 92 levels and the like).
+// chip from half a warp on), 256x256x41 2.16 and 1.79; 128x128x16 with eight
+// sources 1.34 and 1.79, with one 0.44 and 0.26.  The line depends on the grid
+// alone, so that a source's arithmetic does not depend on the batch around it, and
+// lies where neither one source nor eight lose on chip: up to 20 levels from 4000
+// modes, and on the largest grids the boxes that leave too many lanes empty
+// (512x512: 25 to 28, 41 to 46, 81 to 92 levels and the like).
 bool stages_faster(int option, int modes, int nz, const PencilShape& sh) {
     if (modes >= 46000) return (option == 2 && sh.tp > 8 ? 0.95 : 1.0) * pencil_cost(sh) > (modes >= 92000 ? 19.0 : 21.2) * nz;
     return modes >= 4000 && nz <= 20;
@@ -1340,7 +1340,7 @@ static int do_steps(sparc_ctx* c, int nsteps) {
     // the clock on the device, so a captured chunk is valid at any time) and
     // a graph of the remainder: capture and instantiation stay bounded.  Each
     // chunk's last step also writes scr; the call's last step is still the
-    // last to write it.  A magnetic step is some sixty launches, so its chunk is
+    // last to write it.  A magnetic step is about 65 launches, so its chunk is
     // shorter.
     const int kGraphChunk = c->mhd ? 4 : 64;
     if (c->use_graphs && nsteps > kGraphChunk) {

@@ -38,7 +38,7 @@ struct sparc_ctx {
     void* a = nullptr; void* scr = nullptr; void* pml = nullptr; void* scrpml = nullptr;
     void* ybuf = nullptr; void* pbuf = nullptr; void* rbuf = nullptr;
     void* zt = nullptr; void* pt = nullptr;       // T tables
-    float* ftab = nullptr;                        // fused FP32 step: z table [FZ_COUNT][fused_nzp(nz)]
+    float* ftab = nullptr;                        // fused FP32 step: z table [FZ_ROWS][fused_nzp], look-back products
     int use_fused = 0;
     int fused_pencils = 4;                        // modes per CTA of the fused step (autotuned)
     int use_pencil = 0;                           // whole-step kernel of pencil.cu

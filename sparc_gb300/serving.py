@@ -133,7 +133,7 @@ class Pool:
         """Queue nsteps more steps (one step on the flux tube), unless two
         such chunks are still queued: the GPU queues stay short, so the
         streams' priorities decide the order of the pools' work.  A flux-tube
-        step is about a hundred kernels of a graph and takes milliseconds;
+        step is a graph of about 65 kernels and takes milliseconds;
         queuing one at a time keeps cheap pools from waiting behind it.  Returns
         whether steps were queued."""
         import torch
